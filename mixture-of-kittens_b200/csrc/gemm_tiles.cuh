@@ -17,6 +17,7 @@ constexpr int TMEM_COLS = 512;
 constexpr int MODE_ROWS = 0;   // D[row, :] over schedule rows grouped by expert
 constexpr int MODE_WGRAD = 1;  // D[e] = sum over the rows of expert e
 constexpr int kWgradGroup = 8; // weight-gradient tile order: width of a group of the faster-running tile dimension
+constexpr int kRowsGroup = 8;  // rows tile order when an expert's weights do not fit L2: see rows_group()
 
 struct KernelParams {
     const int32_t* tokens_per_expert;
@@ -28,6 +29,7 @@ struct KernelParams {
     int row_begin, row_end;
     int n_blocks;             // rows: N / 256 per output set; wgrad: N / 256
     int m_blocks_w;           // wgrad: M / 256
+    int m_group;              // rows: consecutive m tiles that walk the columns together (0 = 1), see rows_group()
     int k_blocks;             // rows: K steps per operand set
     int n_sets;               // rows: output sets sharing A (1 or 2)
     int k_sets;               // rows: operand sets accumulated into one output (1 or 2)
@@ -52,18 +54,22 @@ struct Tile {
     int accumulate;  // wgrad: add to what is already stored (the expert's rows began in an earlier window)
 };
 
-// Tile t of the static list.  rows: m tile major, then output set, then n tile, so that the tiles running at one
-// time share an expert's weights in L2.  wgrad: expert major, then as described below.  Returns false for tiles
-// without work.
+// Tile t of the static list.  rows: groups of m_group m tiles; in a group output set, then n tile, then the group's m
+// tiles.  With m_group = 1 (m tile major) the tiles running at one time share an expert's weights in L2; rows_group()
+// says when a wider group is taken.  wgrad: expert major, then as described below.  Returns false for tiles without work.
 // (host-callable too: tests/tile_math_host.cu walks the tile lists on the CPU)
 template <int MODE, int BK>
 __host__ __device__ __forceinline__ bool decode_tile(const KernelParams& p, const int* cum, int lo, int hi, int t, Tile& tile) {
     if (MODE == MODE_ROWS) {
-        const int per_m = p.n_blocks * p.n_sets;
-        const int mt = t / per_m;
-        const int rem = t - mt * per_m;
-        tile.set = rem / p.n_blocks;
-        tile.n0 = (rem - tile.set * p.n_blocks) * BN;
+        const int group = max(p.m_group, 1);
+        const int per_group = group * p.n_blocks * p.n_sets;
+        const int g = t / per_group;
+        const int rem = t - g * per_group;
+        const int width = min(group, (hi - lo) / BM - g * group);   // the last group may be narrower
+        const int col = rem / width;
+        const int mt = g * group + (rem - col * width);
+        tile.set = col / p.n_blocks;
+        tile.n0 = (col - tile.set * p.n_blocks) * BN;
         tile.row0 = lo + mt * BM;
         tile.m0 = 0;
         int e = 0;
@@ -225,6 +231,15 @@ inline KernelParams base_params(const GemmProblem& pb) {
     kp.status = pb.status;
     return kp;
 }
+
+// Width of the m-tile groups of a rows form whose tiles read `expert_weight_bytes` of one expert's weights in all.
+// m tile major order (1) reads the activations once and the weights once per m tile, which is free while they stay in
+// L2.  Weights that outgrow it are read from HBM for every m tile: at 235 MB (hidden 4096, intermediate 14336, gate and
+// up) the 74 tiles in flight touch 1 + 74 operand panels.  Groups of 8 make that about 8 + 9.  Measured there, forward +
+// backward of 16384 tokens: 50.5 ms m tile major, 47.5 / 47.0 / 46.8 ms in groups of 4 / 8 / 16.  At 59 MB and below
+// (hidden 7168, intermediate 2048) all widths were within 1 % (m tile major ahead by 0.7 % in MXFP8), so the line is
+// drawn between the two, at half of the 126 MB L2: a line read by SMs of both dies takes room on each.
+inline int rows_group(long long expert_weight_bytes) { return expert_weight_bytes > (63LL << 20) ? kRowsGroup : 1; }
 
 // Launches `kernel` as clusters of two CTAs, as many pairs as can be resident at once (at most one per tile).
 // `resident_pairs` caches the occupancy query per device and kernel instantiation.

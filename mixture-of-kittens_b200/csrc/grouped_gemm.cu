@@ -350,6 +350,7 @@ int launch_rows_gemm(const GemmProblem& pb, const void* A, int K, const void* B0
     kp.n_sets = n_sets;
     kp.D0 = static_cast<bf16*>(D0);
     kp.D1 = static_cast<bf16*>(D1);
+    kp.m_group = rows_group(2LL * n_sets * N * K);
     kp.ldd = N;
     const int window = pb.row_end - pb.row_begin;
     const int max_tiles = (window / BM) * kp.n_blocks * n_sets;
@@ -374,6 +375,7 @@ int launch_gate_up_fused(const GemmProblem& pb, const void* A, int K, const void
     kp.D2 = static_cast<bf16*>(hidden);
     kp.clamp = has_limit ? 1 : 0;
     kp.limit = limit;
+    kp.m_group = rows_group(2LL * 2 * N * K);
     kp.ldd = N;
     const int window = pb.row_end - pb.row_begin;
     return launch<MODE_ROWS, false, true>(a0, b0, a0, b1, kp, (window / BM) * kp.n_blocks, stream);
@@ -395,6 +397,7 @@ int launch_rows_gemm_dual(const GemmProblem& pb, const void* A0, const void* A1,
     kp.k_sets = 2;
     kp.D0 = static_cast<bf16*>(D);
     kp.D1 = nullptr;
+    kp.m_group = rows_group(2LL * 2 * N * K);
     kp.ldd = N;
     const int window = pb.row_end - pb.row_begin;
     return launch<MODE_ROWS, true>(a0, b0, a1, b1, kp, (window / BM) * kp.n_blocks, stream);
@@ -416,6 +419,7 @@ int launch_rows_gemm_f32(const GemmProblem& pb, const void* A, int K, const void
     kp.D0 = reinterpret_cast<bf16*>(D);
     kp.D1 = nullptr;
     kp.out_f32 = 1;
+    kp.m_group = rows_group(2LL * kp.k_sets * N * K);
     kp.ldd = N;
     const int window = pb.row_end - pb.row_begin;
     return launch<MODE_ROWS, false>(a0, b0, a0, b1, kp, (window / BM) * kp.n_blocks, stream);

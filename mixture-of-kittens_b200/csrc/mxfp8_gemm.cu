@@ -454,6 +454,7 @@ int launch_fp8_rows_gemm(const GemmProblem& pb, const Fp8Operand& A, int K, cons
     kp.n_tiles_per_expert = N / 128;
     kp.D0 = static_cast<bf16*>(D0);
     kp.D1 = static_cast<bf16*>(D1);
+    kp.m_group = rows_group(1LL * kp.n_sets * N * K);
     kp.ldd = N;
     return launch<MODE_ROWS>(ms0, ms1, kp, ((pb.row_end - pb.row_begin) / BM) * kp.n_blocks * kp.n_sets, stream);
 }
@@ -475,6 +476,7 @@ int launch_fp8_gate_up_fused(const GemmProblem& pb, const Fp8Operand& A, int K, 
     kp.n_tiles_per_expert = N / 128;
     kp.D0 = nullptr;
     kp.D1 = nullptr;
+    kp.m_group = rows_group(1LL * 2 * N * K);
     kp.ldd = N;
     FusedOut f{};
     f.gate_q = static_cast<uint8_t*>(out.gate_q);
@@ -509,6 +511,7 @@ int launch_fp8_rows_gemm_dual(const GemmProblem& pb, const Fp8Operand& A0, const
     kp.k_sets = 2;
     kp.n_tiles_per_expert = N / 128;
     kp.D0 = static_cast<bf16*>(D);
+    kp.m_group = rows_group(1LL * 2 * N * K);
     kp.ldd = N;
     return launch<MODE_ROWS>(ms0, ms1, kp, ((pb.row_end - pb.row_begin) / BM) * kp.n_blocks, stream);
 }
