@@ -35,7 +35,8 @@ enum {
     MOK_STATUS_SCHEDULE_OVERFLOW = 1u,   /* padded routes exceed schedule_capacity; rows beyond it were dropped */
     MOK_STATUS_BARRIER_TIMEOUT = 2u,     /* a cross-GPU barrier wait ran out */
     MOK_STATUS_PIPELINE_TIMEOUT = 4u,    /* an mbarrier wait inside a GEMM kernel ran out */
-    MOK_STATUS_BAD_SCHEDULE_ENTRY = 8u   /* a schedule row named a peer or token outside the buffers (skipped) */
+    MOK_STATUS_BAD_SCHEDULE_ENTRY = 8u   /* a schedule row named a peer or token outside the buffers (skipped), or the
+                                              schedule claims more rows than the routes padded per expert can fill */
 };
 
 #define MOK_MAX_EP 8

@@ -111,7 +111,10 @@ __global__ void __launch_bounds__(256) dispatch_kernel(PeerTable src, PeerTable 
                                                         int row_begin, int row_end, int ep, int topk, int tokens_per_rank,
                                                         int hidden, uint4* __restrict__ dst, float* __restrict__ row_weight,
                                                         uint32_t* status, const int* __restrict__ row_source,
-                                                        const uint4* __restrict__ staged, int staged_rows, int self_rank) {
+                                                        const uint4* __restrict__ staged, int staged_rows, int self_rank,
+                                                        int covered_rows) {
+    if (*num_tokens > covered_rows && blockIdx.x == 0 && threadIdx.x == 0 && status != nullptr)
+        atomicOr(status, (uint32_t)MOK_STATUS_BAD_SCHEDULE_ENTRY);
     const int hi = min(row_end, *num_tokens);
     const int vec_per_row = hidden / 8;
     const int warps = (gridDim.x * blockDim.x) >> 5;
@@ -235,12 +238,12 @@ int launch_dispatch(const uint64_t* src_ptrs, const uint64_t* weight_ptrs, int e
         dispatch_kernel<true><<<grid, 256, 0, stream>>>(src, wt, w.peer_rank, w.peer_token, w.num_tokens, w.row_begin,
                                                         w.row_end, ep, topk, tokens_per_rank, hidden,
                                                         static_cast<uint4*>(dst), row_weight, w.status, row_source,
-                                                        staged_rows_ptr, n_staged, self);
+                                                        staged_rows_ptr, n_staged, self, w.covered_rows);
     } else {
         dispatch_kernel<false><<<grid, 256, 0, stream>>>(src, wt, w.peer_rank, w.peer_token, w.num_tokens, w.row_begin,
                                                          w.row_end, ep, topk, tokens_per_rank, hidden,
                                                          static_cast<uint4*>(dst), nullptr, w.status, row_source,
-                                                         staged_rows_ptr, n_staged, self);
+                                                         staged_rows_ptr, n_staged, self, w.covered_rows);
     }
     MOK_LAUNCH_CHECK("dispatch_kernel");
     return MOK_OK;

@@ -12,6 +12,7 @@ struct RowWindow {
     const int32_t* num_tokens;
     int row_begin, row_end;
     uint32_t* status;
+    int covered_rows = 0x7fffffff;   // rows the whole call covers; a dispatch reports schedules that claim more
 };
 
 // De-duplicated dispatch (see dedup.cu): the tokens a rank serves, numbered in the order of their first schedule row,

@@ -131,18 +131,21 @@ bool overlap_enabled() {
 // Rows handed from dispatch to the GEMMs to combine in one piece: kMinibatchesPerChunk minibatches, so the caller's
 // minibatch_size sets the hand-over granularity (the default 4096 gives 32768-row chunks, the size that measured best
 // on the DeepSeek-V3-shaped layer).  MOK_CHUNK_ROWS overrides the row count (rounded up to whole minibatches).
-int chunk_rows_for(const mok_layer_args* a) {
+// A window is cut into equal chunks of about that size; one that holds less than one and a half of them stays whole.
+int chunk_rows_for(const mok_layer_args* a, int window_rows) {
     long long rows = static_cast<long long>(kMinibatchesPerChunk) * a->minibatch_size;
     if (const char* v = getenv("MOK_CHUNK_ROWS")) {
         const int r = atoi(v);
         if (r > 0) rows = r;
     }
+    const long long n = (window_rows + rows / 2) / rows;
+    if (n <= 1) return window_rows;
+    rows = (window_rows + n - 1) / n;
     rows = (rows + a->minibatch_size - 1) / a->minibatch_size * a->minibatch_size;
     // never more than ~100 chunks per window: events and launches stay bounded
     const long long min_rows = (a->macrobatch_size / 100 + a->minibatch_size) / a->minibatch_size * a->minibatch_size;
     if (rows < min_rows) rows = min_rows;
-    if (rows > a->macrobatch_size) rows = a->macrobatch_size;
-    return static_cast<int>(rows);
+    return static_cast<int>(rows < window_rows ? rows : window_rows);
 }
 
 int check_common(const mok_layer_args* a, bool fp8 = false) {
@@ -168,7 +171,16 @@ int check_common(const mok_layer_args* a, bool fp8 = false) {
     return MOK_OK;
 }
 
-int num_windows(const mok_layer_args* a) { return (a->schedule_capacity + a->macrobatch_size - 1) / a->macrobatch_size; }
+// Schedule rows that can carry work: every route once, every local expert padded to 256 rows.  The capacity is at least
+// twice the routes of a rank, so launches sized for it find nothing to do in half of the windows and chunks (each costs
+// the host about 5 us and the GPU 2 to 3).  A schedule that was not built by mok_schedule and claims more rows than this
+// sets MOK_STATUS_BAD_SCHEDULE_ENTRY (dispatch_kernel).
+int covered_rows(const mok_layer_args* a) {
+    const long long most = (static_cast<long long>(a->ep_size) * a->num_local_tokens * a->topk + 255LL * a->num_local_experts) / 256 * 256;
+    return static_cast<int>(most < a->schedule_capacity ? most : a->schedule_capacity);
+}
+
+int num_windows(const mok_layer_args* a) { return (covered_rows(a) + a->macrobatch_size - 1) / a->macrobatch_size; }
 
 // rows [begin, end) of the schedule; `base` is the schedule row held by row 0 of the activation buffers
 struct Span {
@@ -179,7 +191,7 @@ Span window_span(const mok_layer_args* a, int w) {
     Span s;
     s.begin = s.base = w * a->macrobatch_size;
     s.end = s.begin + a->macrobatch_size;
-    if (s.end > a->schedule_capacity) s.end = a->schedule_capacity;
+    if (s.end > covered_rows(a)) s.end = covered_rows(a);
     return s;
 }
 
@@ -191,6 +203,7 @@ RowWindow rows_of(const mok_layer_args* a, const Span& s) {
     r.row_begin = s.begin;
     r.row_end = s.end;
     r.status = a->status;
+    if (covered_rows(a) < a->schedule_capacity) r.covered_rows = covered_rows(a);
     return r;
 }
 
@@ -478,7 +491,7 @@ int check_mxfp8_forward_fields(const mok_layer_args* a) {
 template <class Pull, class Compute, class Push>
 int run_chunks(const mok_layer_args* a, const Span& win, bool overlapped, DeviceStreams* d, cudaStream_t main_stream,
                Pull pull, Compute compute, Push push) {
-    const int chunk = chunk_rows_for(a);
+    const int chunk = chunk_rows_for(a, win.end - win.begin);
     const int n = (win.end - win.begin + chunk - 1) / chunk;
     auto span_of = [&](int c) {
         Span s;

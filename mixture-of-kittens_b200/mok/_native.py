@@ -20,7 +20,7 @@ STATUS_BITS = {
     1: "schedule overflow: padded routes exceed schedule_capacity (raise schedule_capacity_multiplier)",
     2: "cross-GPU barrier wait ran out",
     4: "a GEMM pipeline wait ran out",
-    8: "a schedule row named a peer or token outside the buffers",
+    8: "a schedule row named a peer or token outside the buffers, or the schedule claims more rows than its routes fill",
 }
 MAX_EP = 8
 
