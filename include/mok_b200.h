@@ -232,10 +232,11 @@ typedef struct mok_layer_args {
     void *gate_shared, *up_shared, *hidden_shared;   /* [T, I] */
     void *gate_routed, *up_routed, *hidden_routed;   /* [MB, I] */
     void *y_shared;        /* [T, H]  forward out */
-    void *y_routed;        /* [MB, H] forward out */
+    void *y_routed;        /* [MB, H] forward out; NULL: the down projection stores every row straight into its
+                              owner's combine slot and the rows are not kept */
     /* backward outputs / scratch */
     void *d_x_shared;      /* [T, H] */
-    void *d_x_routed;      /* [MB, H] */
+    void *d_x_routed;      /* [MB, H]; NULL: rows and router-weight gradients straight into the owners' slots */
     void *d_gate_shared, *d_up_shared, *d_hidden_shared;   /* [T, I] */
     void *d_gate_routed, *d_up_routed, *d_hidden_routed;   /* [MB, I] */
     void *d_y_routed;      /* [MB, H] */

@@ -20,6 +20,7 @@ constexpr int kWgradGroup = 8; // weight-gradient tile order: width of a group o
 constexpr int kRowsGroup = 8;  // rows tile order when an expert's weights do not fit L2: see rows_group()
 
 struct KernelParams {
+    RowScatter scatter;             // rows forms: output rows go to their owners' slots instead of D0 (see grouped_gemm.cuh)
     const int32_t* tokens_per_expert;
     const int32_t* num_tokens;
     const int32_t* occupied_rows;   // wgrad: see GemmProblem
@@ -174,6 +175,48 @@ __device__ __forceinline__ void store_row_chunk_f32(float* dst, const uint32_t (
     for (int v = 0; v < 8; ++v) out[v] = make_uint4(acc[v * 4], acc[v * 4 + 1], acc[v * 4 + 2], acc[v * 4 + 3]);
 }
 
+// ---- scattered output rows --------------------------------------------------------------------------------
+// A separate combine pass reads and writes every row once more and is bound by HBM (2.6 + 2.6 ms for 270k rows of 7168,
+// forward and backward); here the same 128-byte lines leave the epilogue for their final address, hidden behind the main
+// loop of the next tile, and padding rows are not stored at all.
+// First element of the slot that schedule row `row` belongs to, nullptr for padding rows and for entries outside the
+// buffers (reported).  `first_columns`: the caller owns columns [0, 256) of the row and also delivers its scalar.
+__device__ __forceinline__ bf16* scatter_slot(const RowScatter& s, int row, int row_begin, long long ld, bool first_columns,
+                                              uint32_t* status) {
+    const int peer = s.peer_rank[row], route = s.peer_token[row];
+    if (peer < 0) return nullptr;
+    if (peer >= s.ep || route < 0 || route >= s.routes_per_rank) {
+        if (first_columns && status != nullptr) atomicOr(status, (uint32_t)MOK_STATUS_BAD_SCHEDULE_ENTRY);
+        return nullptr;
+    }
+    if (first_columns && s.row_scalar != nullptr) reinterpret_cast<float*>(s.scalar_ptr[peer])[route] = s.row_scalar[row - row_begin];
+    return reinterpret_cast<bf16*>(s.ptr[peer]) + static_cast<long long>(route) * ld;
+}
+
+// Every lane holds the slot of row `lane` of the warp's 32; spread[it] = slot of the row this lane stores in iteration it
+// of a 64-column store (four rows per iteration, eight lanes per row).
+__device__ __forceinline__ void spread_slots(bf16* mine, bf16* (&spread)[8], int lane) {
+#pragma unroll
+    for (int it = 0; it < 8; ++it)
+        spread[it] = reinterpret_cast<bf16*>(__shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(mine), it * 4 + (lane >> 3)));
+}
+
+// epilogue_store_packed_64cols with an address per row: full 128-byte lines, rows without a slot are left out.
+__device__ __forceinline__ void epilogue_scatter_packed_64cols(uint8_t* warp_patch, const uint4* row_vectors, bf16* const (&slots)[8],
+                                                               int col0, int lane) {
+    uint4* mine = reinterpret_cast<uint4*>(warp_patch + lane * kEpiRowPitch);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) mine[i] = row_vectors[i];
+    __syncwarp();
+    const int seg = lane & 7;
+#pragma unroll
+    for (int it = 0; it < 8; ++it) {
+        const uint4 w = *reinterpret_cast<const uint4*>(warp_patch + (it * 4 + (lane >> 3)) * kEpiRowPitch + seg * 16);
+        if (slots[it] != nullptr) *reinterpret_cast<uint4*>(slots[it] + col0 + seg * 8) = w;
+    }
+    __syncwarp();
+}
+
 // ---------------------------------------------------------------------------------------------------------
 // Host side
 // ---------------------------------------------------------------------------------------------------------
@@ -213,6 +256,14 @@ inline int check_problem(const GemmProblem& pb) {
         return MOK_ERR_INVALID_ARGUMENT;
     if (pb.tokens_per_expert == nullptr && (pb.num_experts != 1 || pb.dense_rows % BM != 0)) return MOK_ERR_INVALID_ARGUMENT;
     if (pb.tokens_per_expert != nullptr && pb.num_tokens == nullptr) return MOK_ERR_INVALID_ARGUMENT;
+    return MOK_OK;
+}
+
+// Destination of a rows form: `D`, or the slots of `scatter` when that is given.
+inline int set_output(KernelParams& kp, void* D, const RowScatter* scatter) {
+    if ((D == nullptr) == (scatter == nullptr)) return MOK_ERR_INVALID_ARGUMENT;
+    kp.D0 = static_cast<bf16*>(D);
+    if (scatter != nullptr) kp.scatter = *scatter;
     return MOK_OK;
 }
 

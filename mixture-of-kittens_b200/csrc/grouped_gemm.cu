@@ -215,6 +215,9 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_const
             if (!decode_tile<MODE, BK>(p, cum, lo, hi, t, tile)) continue;
             const int acc = iter & 1;
             const uint32_t acc_phase = (iter >> 1) & 1u;
+            const bool scattered = MODE == MODE_ROWS && !FUSED && p.scatter.peer_rank != nullptr;
+            bf16* slot = nullptr;   // looked up while the tile is still being accumulated
+            if (scattered) slot = scatter_slot(p.scatter, tile.row0 + row_in_tile, p.row_begin, p.ldd, tile.n0 == 0, p.status);
             ok = mbar_wait(bar_tmem_full + 8 * acc, acc_phase, abort_flag, p.status);
             if (!ok) break;
             tc_fence_after_sync();
@@ -263,6 +266,20 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_const
                     epilogue_store_packed_64cols(patch, gate, p.D0 + first + c * 64, p.ldd, lane);
                     epilogue_store_packed_64cols(patch, up, p.D1 + first + c * 64, p.ldd, lane);
                     epilogue_store_packed_64cols(patch, hid, p.D2 + first + c * 64, p.ldd, lane);
+                }
+            } else if (scattered) {
+                bf16* slots[8];
+                spread_slots(slot, slots, lane);
+#pragma unroll 1
+                for (int c = 0; c < BN / 64; ++c) {
+                    uint32_t v0[32], v1[32];
+                    tmem_ld_32x32(taddr + c * 64, v0);
+                    tmem_ld_32x32(taddr + c * 64 + 32, v1);
+                    tmem_ld_wait();
+                    uint4 packed[8];
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) { packed[i] = pack8_bf16(&v0[8 * i]); packed[4 + i] = pack8_bf16(&v1[8 * i]); }
+                    epilogue_scatter_packed_64cols(patch, packed, slots, tile.n0 + c * 64, lane);
                 }
             } else
 #pragma unroll 1
@@ -330,7 +347,7 @@ int launch(const CUtensorMap& a0, const CUtensorMap& b0, const CUtensorMap& a1, 
 }  // namespace
 
 int launch_rows_gemm(const GemmProblem& pb, const void* A, int K, const void* B0, const void* B1, void* D0, void* D1,
-                     int N, bool b_is_kn, cudaStream_t stream) {
+                     int N, bool b_is_kn, cudaStream_t stream, const RowScatter* scatter) {
     int rc = check_problem(pb);
     if (rc != MOK_OK) return rc;
     if (K <= 0 || N <= 0 || K % BK != 0 || N % BN != 0) return MOK_ERR_INVALID_ARGUMENT;
@@ -348,7 +365,7 @@ int launch_rows_gemm(const GemmProblem& pb, const void* A, int K, const void* B0
     kp.n_blocks = N / BN;
     kp.k_blocks = K / BK;
     kp.n_sets = n_sets;
-    kp.D0 = static_cast<bf16*>(D0);
+    if ((rc = set_output(kp, D0, scatter)) != MOK_OK || (scatter != nullptr && n_sets != 1)) return MOK_ERR_INVALID_ARGUMENT;
     kp.D1 = static_cast<bf16*>(D1);
     kp.m_group = rows_group(2LL * n_sets * N * K);
     kp.ldd = N;
@@ -382,7 +399,7 @@ int launch_gate_up_fused(const GemmProblem& pb, const void* A, int K, const void
 }
 
 int launch_rows_gemm_dual(const GemmProblem& pb, const void* A0, const void* A1, int K, const void* B0, const void* B1,
-                          void* D, int N, cudaStream_t stream) {
+                          void* D, int N, cudaStream_t stream, const RowScatter* scatter) {
     int rc = check_problem(pb);
     if (rc != MOK_OK) return rc;
     if (K <= 0 || N <= 0 || K % BK != 0 || N % BN != 0) return MOK_ERR_INVALID_ARGUMENT;
@@ -395,7 +412,7 @@ int launch_rows_gemm_dual(const GemmProblem& pb, const void* A0, const void* A1,
     kp.n_blocks = N / BN;
     kp.k_blocks = K / BK;
     kp.k_sets = 2;
-    kp.D0 = static_cast<bf16*>(D);
+    if ((rc = set_output(kp, D, scatter)) != MOK_OK) return rc;
     kp.D1 = nullptr;
     kp.m_group = rows_group(2LL * 2 * N * K);
     kp.ldd = N;

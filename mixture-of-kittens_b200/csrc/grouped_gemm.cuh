@@ -22,10 +22,23 @@ struct GemmProblem {
     uint32_t* status = nullptr;
 };
 
+// Output rows of a rows form that are stored into the token owners' slot buffers: row r goes to
+// ptr[peer_rank[r]][peer_token[r], :] (local or peer memory; padding rows nowhere), and with row_scalar its fp32 value
+// row_scalar[r - row_begin] to scalar_ptr[peer_rank[r]][peer_token[r]].  One GEMM epilogue then does what a plain store
+// and a combine pass over the stored rows would do.
+struct RowScatter {
+    uint64_t ptr[MOK_MAX_EP] = {};
+    uint64_t scalar_ptr[MOK_MAX_EP] = {};
+    const int32_t* peer_rank = nullptr;    // [schedule rows]; nullptr = not scattered
+    const int32_t* peer_token = nullptr;
+    const float* row_scalar = nullptr;
+    int ep = 0, routes_per_rank = 0;
+};
+
 // D_s[row, :] = A[row, :K] * B_s[e]^T for s < n_sets (two sets share A: gate and up projections).
-// b_is_kn = false: B_s is [E, N, K];  true: B_s is [E, K, N].
+// With `scatter` (one set only) D0 is nullptr and the rows go to their slots.  b_is_kn = false: B_s is [E, N, K];  true: B_s is [E, K, N].
 int launch_rows_gemm(const GemmProblem& pb, const void* A, int K, const void* B0, const void* B1, void* D0, void* D1,
-                     int N, bool b_is_kn, cudaStream_t stream);
+                     int N, bool b_is_kn, cudaStream_t stream, const RowScatter* scatter = nullptr);
 
 // Forward gate and up projections with the SwiGLU in the epilogue: gate = A * Wg[e]^T, up = A * Wu[e]^T (both stored as
 // bf16 [rows, N]) and hidden = silu(gate) * up computed from the stored (rounded) values, optionally clamped.
@@ -34,7 +47,7 @@ int launch_gate_up_fused(const GemmProblem& pb, const void* A, int K, const void
 
 // D[row, :] = A0[row, :K] * B0[e] + A1[row, :K] * B1[e] with B_s stored [E, K, N] (gate+up input gradient).
 int launch_rows_gemm_dual(const GemmProblem& pb, const void* A0, const void* A1, int K, const void* B0, const void* B1,
-                          void* D, int N, cudaStream_t stream);
+                          void* D, int N, cudaStream_t stream, const RowScatter* scatter = nullptr);
 
 // D[e] [M, N] (+)= A[rows_e, M]^T * B[rows_e, N]; accumulates when expert e's rows began before row_begin.
 // out_f32: D is fp32 and is overwritten (single-window problems only).

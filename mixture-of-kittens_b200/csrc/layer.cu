@@ -217,6 +217,8 @@ const bf16* rows_bf16(const void* buffer, const Span& s, int row_elems) {
     return at_row(static_cast<const bf16*>(buffer), s, row_elems);
 }
 
+bf16* rows_or_null(void* buffer, const Span& s, int row_elems) { return buffer ? rows_bf16(buffer, s, row_elems) : nullptr; }
+
 GemmProblem routed_problem(const mok_layer_args* a, const Span& s) {
     GemmProblem p;
     p.tokens_per_expert = a->tokens_per_expert;
@@ -331,6 +333,21 @@ int dispatch_d_y(const mok_layer_args* a, const Span& s, float* row_weight, int 
         return staged_dispatch(a, a->d_y_ptrs, a->router_weight_ptrs, a->staged_d_y, staging, s, dst, at_row(row_weight, s, 1), ctas, st);
     return launch_dispatch(a->d_y_ptrs, a->router_weight_ptrs, a->ep_size, rows_of(a, s), a->topk, a->num_local_tokens, a->hidden,
                            dst, at_row(row_weight, s, 1), ctas, st);
+}
+
+// Slots of a combine that the GEMM epilogue performs itself (the caller gave no buffer for the rows).
+int slots_of(const mok_layer_args* a, const uint64_t* ptrs, const uint64_t* scalar_ptrs, const float* row_scalar, RowScatter* out) {
+    for (int i = 0; i < a->ep_size; ++i) {
+        if (ptrs[i] == 0 || (ptrs[i] & 15u) != 0 || (row_scalar != nullptr && scalar_ptrs[i] == 0)) return MOK_ERR_INVALID_ARGUMENT;
+        out->ptr[i] = ptrs[i];
+        if (row_scalar != nullptr) out->scalar_ptr[i] = scalar_ptrs[i];
+    }
+    out->peer_rank = a->peer_rank;
+    out->peer_token = a->peer_token_idx;
+    out->row_scalar = row_scalar;
+    out->ep = a->ep_size;
+    out->routes_per_rank = a->num_local_tokens * a->topk;
+    return MOK_OK;
 }
 
 int gate_up_hidden(const mok_layer_args* a, const Span& s, cudaStream_t st) {
@@ -546,7 +563,7 @@ int run_chunks(const mok_layer_args* a, const Span& win, bool overlapped, Device
 extern "C" int mok_moe_forward_bf16(const mok_layer_args* a, mok_stream_t stream) {
     using namespace mok;
     MOK_TRY(check_common(a));
-    if (!a->combine_ptrs || !a->w_routed_down || !a->y_routed) return MOK_ERR_INVALID_ARGUMENT;
+    if (!a->combine_ptrs || !a->w_routed_down) return MOK_ERR_INVALID_ARGUMENT;
     if (a->w_shared_gate && (!a->w_shared_down || !a->y_shared)) return MOK_ERR_INVALID_ARGUMENT;
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
     Staging x_staging, d_y_staging;   // how far the de-duplicated tokens of x / d_y have been staged in this call
@@ -567,10 +584,13 @@ extern "C" int mok_moe_forward_bf16(const mok_layer_args* a, mok_stream_t stream
             [&](const Span& c, int ctas, cudaStream_t st) { return dispatch_x(a, c, ctas, st, &x_staging); },
             [&](const Span& c, cudaStream_t st) {
                 MOK_TRY(gate_up_hidden(a, c, st));
+                RowScatter slots;
+                if (a->y_routed == nullptr) MOK_TRY(slots_of(a, a->combine_ptrs, nullptr, nullptr, &slots));
                 return launch_rows_gemm(routed_problem(a, c), rows_bf16(a->hidden_routed, c, I), I, a->w_routed_down, nullptr,
-                                        rows_bf16(a->y_routed, c, H), nullptr, H, false, st);
+                                        rows_or_null(a->y_routed, c, H), nullptr, H, false, st, a->y_routed ? nullptr : &slots);
             },
             [&](const Span& c, int ctas, cudaStream_t st) {
+                if (a->y_routed == nullptr) return static_cast<int>(MOK_OK);
                 return launch_combine(a->combine_ptrs, nullptr, a->ep_size, rows_of(a, c), a->topk, a->num_local_tokens, H,
                                       rows_bf16(a->y_routed, c, H), nullptr, ctas, st);
             }));
@@ -600,7 +620,7 @@ extern "C" int mok_moe_backward_bf16(const mok_layer_args* a, mok_stream_t strea
     MOK_TRY(check_common(a));
     if (!a->d_y_ptrs || !a->d_x_routed_ptrs || !a->router_weight_ptrs || !a->d_router_weight_ptrs || !a->w_routed_down)
         return MOK_ERR_INVALID_ARGUMENT;
-    if (!a->d_x_routed || !a->d_gate_routed || !a->d_up_routed || !a->d_hidden_routed || !a->d_y_routed ||
+    if (!a->d_gate_routed || !a->d_up_routed || !a->d_hidden_routed || !a->d_y_routed ||
         !a->d_w_routed_gate || !a->d_w_routed_up || !a->d_w_routed_down || !a->row_scratch)
         return MOK_ERR_INVALID_ARGUMENT;
     const bool shared = a->w_shared_gate != nullptr;
@@ -644,10 +664,15 @@ extern "C" int mok_moe_backward_bf16(const mok_layer_args* a, mok_stream_t strea
                                           rows_bf16(a->d_hidden_routed, c, I), rows_bf16(a->d_gate_routed, c, I),
                                           rows_bf16(a->d_up_routed, c, I), a->num_tokens, 0, c.begin, c.end, I, clamp,
                                           a->swiglu_limit, at_row(row_weight, c, 1), at_row(row_grad, c, 1), st));
+                RowScatter slots;
+                if (a->d_x_routed == nullptr)
+                    MOK_TRY(slots_of(a, a->d_x_routed_ptrs, a->d_router_weight_ptrs, at_row(row_grad, c, 1), &slots));
                 return launch_rows_gemm_dual(p, rows_bf16(a->d_gate_routed, c, I), rows_bf16(a->d_up_routed, c, I), I,
-                                             a->w_routed_gate, a->w_routed_up, rows_bf16(a->d_x_routed, c, H), H, st);
+                                             a->w_routed_gate, a->w_routed_up, rows_or_null(a->d_x_routed, c, H), H, st,
+                                             a->d_x_routed ? nullptr : &slots);
             },
             [&](const Span& c, int ctas, cudaStream_t st) {
+                if (a->d_x_routed == nullptr) return static_cast<int>(MOK_OK);
                 return launch_combine(a->d_x_routed_ptrs, a->d_router_weight_ptrs, a->ep_size, rows_of(a, c), a->topk, T, H,
                                       rows_bf16(a->d_x_routed, c, H), at_row(row_grad, c, 1), ctas, st);
             }));
@@ -676,7 +701,7 @@ extern "C" int mok_moe_forward_mxfp8(const mok_layer_args* a, mok_stream_t strea
     using namespace mok;
     MOK_TRY(check_common(a, true));
     MOK_TRY(check_mxfp8_forward_fields(a));
-    if (!a->combine_ptrs || !a->w_down_fp8 || !a->w_down_sc || !a->y_routed) return MOK_ERR_INVALID_ARGUMENT;
+    if (!a->combine_ptrs || !a->w_down_fp8 || !a->w_down_sc) return MOK_ERR_INVALID_ARGUMENT;
     if (a->w_shared_gate && (!a->w_shared_down || !a->y_shared)) return MOK_ERR_INVALID_ARGUMENT;
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
     Staging x_staging, d_y_staging;   // how far the de-duplicated tokens of x / d_y have been staged in this call
@@ -698,10 +723,13 @@ extern "C" int mok_moe_forward_mxfp8(const mok_layer_args* a, mok_stream_t strea
             [&](const Span& c, int ctas, cudaStream_t st) { return dispatch_x(a, c, ctas, st, &x_staging); },
             [&](const Span& c, cudaStream_t st) {
                 MOK_TRY(gate_up_hidden_mxfp8(a, c, st));
+                RowScatter slots;
+                if (a->y_routed == nullptr) MOK_TRY(slots_of(a, a->combine_ptrs, nullptr, nullptr, &slots));
                 return launch_fp8_rows_gemm(routed_problem(a, c), act_rows(a, a->hidden_fp8, a->hidden_sc, I, c), I, wd, nullptr,
-                                            rows_bf16(a->y_routed, c, H), nullptr, H, st);
+                                            rows_or_null(a->y_routed, c, H), nullptr, H, st, a->y_routed ? nullptr : &slots);
             },
             [&](const Span& c, int ctas, cudaStream_t st) {
+                if (a->y_routed == nullptr) return static_cast<int>(MOK_OK);
                 return launch_combine(a->combine_ptrs, nullptr, a->ep_size, rows_of(a, c), a->topk, a->num_local_tokens, H,
                                       rows_bf16(a->y_routed, c, H), nullptr, ctas, st);
             }));
@@ -733,7 +761,7 @@ extern "C" int mok_moe_backward_mxfp8(const mok_layer_args* a, mok_stream_t stre
     if (!a->d_y_ptrs || !a->d_x_routed_ptrs || !a->router_weight_ptrs || !a->d_router_weight_ptrs) return MOK_ERR_INVALID_ARGUMENT;
     if (!a->w_gate_t_fp8 || !a->w_gate_t_sc || !a->w_up_t_fp8 || !a->w_up_t_sc || !a->w_down_t_fp8 || !a->w_down_t_sc)
         return MOK_ERR_INVALID_ARGUMENT;
-    if (!a->d_x_routed || !a->d_gate_routed || !a->d_up_routed || !a->d_hidden_routed || !a->d_y_routed || !a->d_w_routed_gate ||
+    if (!a->d_gate_routed || !a->d_up_routed || !a->d_hidden_routed || !a->d_y_routed || !a->d_w_routed_gate ||
         !a->d_w_routed_up || !a->d_w_routed_down || !a->row_scratch)
         return MOK_ERR_INVALID_ARGUMENT;
     if (!a->d_y_fp8 || !a->d_y_sc || !a->d_y_fp8_t || !a->d_y_sc_t || !a->d_gate_fp8 || !a->d_gate_sc || !a->d_up_fp8 ||
@@ -778,6 +806,9 @@ extern "C" int mok_moe_backward_mxfp8(const mok_layer_args* a, mok_stream_t stre
             [&](const Span& c, cudaStream_t st) {
                 const GemmProblem p = routed_problem(a, c);
                 const long long off = c.begin - c.base;
+                RowScatter slots;
+                if (a->d_x_routed == nullptr)
+                    MOK_TRY(slots_of(a, a->d_x_routed_ptrs, a->d_router_weight_ptrs, at_row(row_grad, c, 1), &slots));
                 MOK_TRY(quantize_span(a, c, a->d_y_routed, H, a->d_y_fp8, a->d_y_sc, a->d_y_fp8_t, a->d_y_sc_t, st));
                 MOK_TRY(launch_fp8_rows_gemm(p, act_rows(a, a->d_y_fp8, a->d_y_sc, H, c), H, wd_t, nullptr,
                                              rows_bf16(a->d_hidden_routed, c, I), nullptr, I, st));
@@ -796,7 +827,7 @@ extern "C" int mok_moe_backward_mxfp8(const mok_layer_args* a, mok_stream_t stre
                                                c.begin, c.end, st));
                     return launch_fp8_rows_gemm_dual(p, act_rows(a, a->d_gate_fp8, a->d_gate_sc, I, c),
                                                      act_rows(a, a->d_up_fp8, a->d_up_sc, I, c), I, wg_t, wu_t,
-                                                     rows_bf16(a->d_x_routed, c, H), H, st);
+                                                     rows_or_null(a->d_x_routed, c, H), H, st, a->d_x_routed ? nullptr : &slots);
                 }
                 // the saved gate / up are e4m3: expand them (exactly) into the bf16 scratch the SwiGLU backward reads
                 MOK_TRY(launch_dequantize_rows(static_cast<const uint8_t*>(a->gate_fp8) + off * I,
@@ -813,9 +844,10 @@ extern "C" int mok_moe_backward_mxfp8(const mok_layer_args* a, mok_stream_t stre
                 MOK_TRY(quantize_span(a, c, a->d_up_routed, I, a->d_up_fp8, a->d_up_sc, a->d_up_fp8_t, a->d_up_sc_t, st));
                 return launch_fp8_rows_gemm_dual(p, act_rows(a, a->d_gate_fp8, a->d_gate_sc, I, c),
                                                  act_rows(a, a->d_up_fp8, a->d_up_sc, I, c), I, wg_t, wu_t,
-                                                 rows_bf16(a->d_x_routed, c, H), H, st);
+                                                 rows_or_null(a->d_x_routed, c, H), H, st, a->d_x_routed ? nullptr : &slots);
             },
             [&](const Span& c, int ctas, cudaStream_t st) {
+                if (a->d_x_routed == nullptr) return static_cast<int>(MOK_OK);
                 return launch_combine(a->d_x_routed_ptrs, a->d_router_weight_ptrs, a->ep_size, rows_of(a, c), a->topk, T, H,
                                       rows_bf16(a->d_x_routed, c, H), at_row(row_grad, c, 1), ctas, st);
             }));

@@ -304,6 +304,9 @@ mxfp8_gemm_kernel(const __grid_constant__ MapSet ms0, const __grid_constant__ Ma
         for (int t = pair; t < num_tiles && ok; t += num_pairs) {
             Tile tile;
             if (!decode_tile<MODE, BK>(p, cum, lo, hi, t, tile)) continue;
+            const bool scattered = MODE == MODE_ROWS && !FUSED && p.scatter.peer_rank != nullptr;
+            bf16* slot = nullptr;   // looked up while the tile is still being accumulated
+            if (scattered) slot = scatter_slot(p.scatter, tile.row0 + row_in_tile, p.row_begin, p.ldd, tile.n0 == 0, p.status);
             ok = mbar_wait(bar_tmem_full, iter & 1u, abort_flag, p.status);
             if (!ok) break;
             tc_fence_after_sync();
@@ -350,6 +353,12 @@ mxfp8_gemm_kernel(const __grid_constant__ MapSet ms0, const __grid_constant__ Ma
                     const long long R0 = tile.row0 - p.row_begin + cta_rank * BM_CTA + quarter * 32;
                     if (f.clamp) fused_gate_up_epilogue<true>(f, packed, patch, R0, tile.n0 / 2, quarter, lane);
                     else fused_gate_up_epilogue<false>(f, packed, patch, R0, tile.n0 / 2, quarter, lane);
+                } else if (scattered) {
+                    bf16* slots[8];
+                    spread_slots(slot, slots, lane);
+#pragma unroll
+                    for (int c = 0; c < BN / 64; ++c)
+                        epilogue_scatter_packed_64cols(patch, &packed[c * 8], slots, tile.n0 + c * 64, lane);
                 } else {
 #pragma unroll
                     for (int c = 0; c < BN / 64; ++c)
@@ -440,7 +449,7 @@ int launch(const MapSet& ms0, const MapSet& ms1, KernelParams kp, int max_tiles,
 }  // namespace
 
 int launch_fp8_rows_gemm(const GemmProblem& pb, const Fp8Operand& A, int K, const Fp8Operand& B0, const Fp8Operand* B1,
-                         void* D0, void* D1, int N, cudaStream_t stream) {
+                         void* D0, void* D1, int N, cudaStream_t stream, const RowScatter* scatter) {
     int rc = check_problem(pb);
     if (rc != MOK_OK) return rc;
     if (K <= 0 || N <= 0 || K % BK != 0 || N % BN != 0) return MOK_ERR_INVALID_ARGUMENT;
@@ -452,7 +461,7 @@ int launch_fp8_rows_gemm(const GemmProblem& pb, const Fp8Operand& A, int K, cons
     kp.k_blocks = K / BK;
     kp.n_sets = B1 ? 2 : 1;
     kp.n_tiles_per_expert = N / 128;
-    kp.D0 = static_cast<bf16*>(D0);
+    if ((rc = set_output(kp, D0, scatter)) != MOK_OK || (scatter != nullptr && B1 != nullptr)) return MOK_ERR_INVALID_ARGUMENT;
     kp.D1 = static_cast<bf16*>(D1);
     kp.m_group = rows_group(1LL * kp.n_sets * N * K);
     kp.ldd = N;
@@ -498,7 +507,7 @@ int launch_fp8_gate_up_fused(const GemmProblem& pb, const Fp8Operand& A, int K, 
 }
 
 int launch_fp8_rows_gemm_dual(const GemmProblem& pb, const Fp8Operand& A0, const Fp8Operand& A1, int K, const Fp8Operand& B0,
-                              const Fp8Operand& B1, void* D, int N, cudaStream_t stream) {
+                              const Fp8Operand& B1, void* D, int N, cudaStream_t stream, const RowScatter* scatter) {
     int rc = check_problem(pb);
     if (rc != MOK_OK) return rc;
     if (K <= 0 || N <= 0 || K % BK != 0 || N % BN != 0) return MOK_ERR_INVALID_ARGUMENT;
@@ -510,7 +519,7 @@ int launch_fp8_rows_gemm_dual(const GemmProblem& pb, const Fp8Operand& A0, const
     kp.k_blocks = K / BK;
     kp.k_sets = 2;
     kp.n_tiles_per_expert = N / 128;
-    kp.D0 = static_cast<bf16*>(D);
+    if ((rc = set_output(kp, D, scatter)) != MOK_OK) return rc;
     kp.m_group = rows_group(1LL * 2 * N * K);
     kp.ldd = N;
     return launch<MODE_ROWS>(ms0, ms1, kp, ((pb.row_end - pb.row_begin) / BM) * kp.n_blocks, stream);

@@ -16,13 +16,13 @@ struct Fp8Operand {
     long long scale_row_tile_stride = 0;   // bytes between the scale tiles of consecutive row tiles
 };
 
-// D_s[row, :] = A[row, :K] * B_s[e]^T  (s < 2 when B1 is given); B_s is [E, N, K].  bf16 output.
+// D_s[row, :] = A[row, :K] * B_s[e]^T  (s < 2 when B1 is given); B_s is [E, N, K].  bf16 output.  `scatter` as in grouped_gemm.cuh.
 int launch_fp8_rows_gemm(const GemmProblem& pb, const Fp8Operand& A, int K, const Fp8Operand& B0, const Fp8Operand* B1,
-                         void* D0, void* D1, int N, cudaStream_t stream);
+                         void* D0, void* D1, int N, cudaStream_t stream, const RowScatter* scatter = nullptr);
 
 // D[row, :] = A0[row, :K] * B0[e]^T + A1[row, :K] * B1[e]^T.
 int launch_fp8_rows_gemm_dual(const GemmProblem& pb, const Fp8Operand& A0, const Fp8Operand& A1, int K, const Fp8Operand& B0,
-                              const Fp8Operand& B1, void* D, int N, cudaStream_t stream);
+                              const Fp8Operand& B1, void* D, int N, cudaStream_t stream, const RowScatter* scatter = nullptr);
 
 // Outputs of the fused gate / up projection: every pointer addresses the window's first row (the transposed matrix: its
 // column), scale pointers its first 128-row tile.  Same conventions as launch_quantize_rows (mxfp8.cuh).

@@ -141,7 +141,7 @@ def _keep(args: LayerArgs, **arrays):
 
 def _set_ptrs(args: LayerArgs, **tensors) -> None:
     for field, tensor in tensors.items():
-        setattr(args, field, None if tensor is None else tensor.data_ptr())
+        setattr(args, field, None if tensor is None else tensor.data_ptr() or None)
 
 
 def _new_fp8(like: torch.Tensor, rows: int, cols: int):
@@ -426,12 +426,14 @@ def dispatch_mlp_swiglu_combine_fwd_bf16(
     dedup_unique_peer: torch.Tensor | None = None,
     dedup_unique_token: torch.Tensor | None = None,
     dedup_unique_before: torch.Tensor | None = None,
+    skip_routed_output: bool = False,
 ) -> tuple[torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor,
            torch.Tensor]:
     """BF16 forward: dispatch, routed + shared SwiGLU FFN, combine into the owners' slot buffers.
 
     Outputs: x_routed [MB,H], gate_shared [T,I], gate_routed [MB,I], up_shared, up_routed, hidden_shared,
              hidden_routed, y_shared [T,H], y_routed [MB,H]  (all bfloat16)
+    With skip_routed_output the down projection stores its rows straight into the combine slots and y_routed is [0,H].
     """
     T, H, I, E = _check_activation_dims(x, w_shared_gate, w_routed_gate)
     _check_layer_scalars(topk, swiglu_limit, num_comm_sms, macrobatch_size, minibatch_size)
@@ -452,7 +454,7 @@ def dispatch_mlp_swiglu_combine_fwd_bf16(
                             ("w_shared_down", w_shared_down), ("w_routed_down", w_routed_down)))
 
     new = lambda r, c: x.new_empty((r, c))  # noqa: E731
-    x_routed, y_routed = new(macrobatch_size, H), new(macrobatch_size, H)
+    x_routed, y_routed = new(macrobatch_size, H), new(0 if skip_routed_output else macrobatch_size, H)
     gate_shared, up_shared, hidden_shared = new(T, I), new(T, I), new(T, I)
     gate_routed, up_routed, hidden_routed = new(macrobatch_size, I), new(macrobatch_size, I), new(macrobatch_size, I)
     y_shared = torch.empty_like(x)
@@ -465,7 +467,7 @@ def dispatch_mlp_swiglu_combine_fwd_bf16(
     a.num_tokens, a.tokens_per_expert = num_tokens.data_ptr(), tokens_per_expert.data_ptr()
     a.w_shared_gate, a.w_shared_up, a.w_shared_down = w_shared_gate.data_ptr(), w_shared_up.data_ptr(), w_shared_down.data_ptr()
     a.w_routed_gate, a.w_routed_up, a.w_routed_down = w_routed_gate.data_ptr(), w_routed_up.data_ptr(), w_routed_down.data_ptr()
-    a.x_routed, a.y_routed, a.y_shared = x_routed.data_ptr(), y_routed.data_ptr(), y_shared.data_ptr()
+    a.x_routed, a.y_routed, a.y_shared = x_routed.data_ptr(), y_routed.data_ptr() or None, y_shared.data_ptr()
     a.gate_shared, a.up_shared, a.hidden_shared = gate_shared.data_ptr(), up_shared.data_ptr(), hidden_shared.data_ptr()
     a.gate_routed, a.up_routed, a.hidden_routed = gate_routed.data_ptr(), up_routed.data_ptr(), hidden_routed.data_ptr()
     _staging = _attach_dedup(a, x, cap, ('x',), True, dedup_row_source, dedup_unique_peer, dedup_unique_token,
@@ -576,6 +578,7 @@ def dispatch_mlp_swiglu_combine_bwd_bf16(
     dedup_unique_peer: torch.Tensor | None = None,
     dedup_unique_token: torch.Tensor | None = None,
     dedup_unique_before: torch.Tensor | None = None,
+    skip_routed_output: bool = False,
 ) -> tuple[torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor,
            torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor]:
     """BF16 backward of the layer.
@@ -583,7 +586,8 @@ def dispatch_mlp_swiglu_combine_bwd_bf16(
     Outputs: d_x_shared [T,H], d_x_routed [MB,H], d_gate_shared [T,I], d_gate_routed [MB,I], d_up_shared,
              d_up_routed, d_hidden_shared, d_hidden_routed, d_y_routed [MB,H], d_w_shared_gate [I,H],
              d_w_routed_gate [E,I,H], d_w_shared_up, d_w_routed_up, d_w_shared_down [H,I], d_w_routed_down [E,H,I]
-    The routed input gradients and router-weight gradients land in the owners' symmetric buffers.
+    The routed input gradients and router-weight gradients land in the owners' symmetric buffers; with
+    skip_routed_output the GEMM stores them there itself and d_x_routed is [0,H].
     """
     T, H, I, E = _check_activation_dims(x, w_shared_gate, w_routed_gate)
     _check_layer_scalars(topk, swiglu_limit, num_comm_sms, macrobatch_size, minibatch_size)
@@ -615,7 +619,7 @@ def dispatch_mlp_swiglu_combine_bwd_bf16(
                             ("w_shared_down", w_shared_down), ("w_routed_down", w_routed_down)))
 
     new = lambda *shape: x.new_empty(shape)  # noqa: E731
-    d_x_shared, d_x_routed, d_y_routed = new(T, H), new(MB, H), new(MB, H)
+    d_x_shared, d_x_routed, d_y_routed = new(T, H), new(0 if skip_routed_output else MB, H), new(MB, H)
     d_gate_shared, d_up_shared, d_hidden_shared = new(T, I), new(T, I), new(T, I)
     d_gate_routed, d_up_routed, d_hidden_routed = new(MB, I), new(MB, I), new(MB, I)
     d_w_shared_gate, d_w_shared_up, d_w_shared_down = new(I, H), new(I, H), new(H, I)
@@ -634,7 +638,7 @@ def dispatch_mlp_swiglu_combine_bwd_bf16(
     a.x_routed = x_routed.data_ptr()
     a.gate_shared, a.up_shared, a.hidden_shared = gate_shared.data_ptr(), up_shared.data_ptr(), hidden_shared.data_ptr()
     a.gate_routed, a.up_routed, a.hidden_routed = gate_routed.data_ptr(), up_routed.data_ptr(), hidden_routed.data_ptr()
-    a.d_x_shared, a.d_x_routed, a.d_y_routed = d_x_shared.data_ptr(), d_x_routed.data_ptr(), d_y_routed.data_ptr()
+    a.d_x_shared, a.d_x_routed, a.d_y_routed = d_x_shared.data_ptr(), d_x_routed.data_ptr() or None, d_y_routed.data_ptr()
     a.d_gate_shared, a.d_up_shared, a.d_hidden_shared = d_gate_shared.data_ptr(), d_up_shared.data_ptr(), d_hidden_shared.data_ptr()
     a.d_gate_routed, a.d_up_routed, a.d_hidden_routed = d_gate_routed.data_ptr(), d_up_routed.data_ptr(), d_hidden_routed.data_ptr()
     a.d_w_shared_gate, a.d_w_shared_up, a.d_w_shared_down = d_w_shared_gate.data_ptr(), d_w_shared_up.data_ptr(), d_w_shared_down.data_ptr()
@@ -726,12 +730,14 @@ def dispatch_mlp_swiglu_combine_fwd_mxfp8(
     dedup_unique_peer: torch.Tensor | None = None,
     dedup_unique_token: torch.Tensor | None = None,
     dedup_unique_before: torch.Tensor | None = None,
+    skip_routed_output: bool = False,
 ) -> tuple[torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor,
            torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor]:
     """MXFP8 forward (routed experts in e4m3 with e8m0 block scales, shared expert in bf16).
 
     Outputs: x_fp8_t_routed [H,MB], x_sc_t_routed, gate_shared, gate_fp8_routed [MB,I], gate_sc_routed, up_shared,
              up_fp8_routed, up_sc_routed, hidden_shared, hidden_fp8_t_routed [I,MB], hidden_sc_t_routed, y_shared, y_routed
+    (y_routed is [0,H] with skip_routed_output: the rows go straight into the combine slots)
     """
     T, H, I, E = _check_activation_dims(x, w_shared_gate, w_routed_gate)
     _check_layer_scalars(topk, swiglu_limit, num_comm_sms, macrobatch_size, minibatch_size)
@@ -756,7 +762,8 @@ def dispatch_mlp_swiglu_combine_fwd_mxfp8(
     gate_q, gate_sc = _new_fp8(x, MB, I)
     up_q, up_sc = _new_fp8(x, MB, I)
     hid_t, hid_t_sc = _new_fp8(x, I, MB)
-    gate_shared, up_shared, hidden_shared, y_shared, y_routed = new(T, I), new(T, I), new(T, I), new(T, H), new(MB, H)
+    gate_shared, up_shared, hidden_shared, y_shared = new(T, I), new(T, I), new(T, I), new(T, H)
+    y_routed = new(0 if skip_routed_output else MB, H)
     scratch = dict(x_routed=new(MB, H), gate_routed=new(MB, I), up_routed=new(MB, I), hidden_routed=new(MB, I))
     x_q, x_sc = _new_fp8(x, MB, H)
     hid_q, hid_sc = _new_fp8(x, MB, I)
@@ -900,6 +907,7 @@ def dispatch_mlp_swiglu_combine_bwd_mxfp8(
     dedup_unique_peer: torch.Tensor | None = None,
     dedup_unique_token: torch.Tensor | None = None,
     dedup_unique_before: torch.Tensor | None = None,
+    skip_routed_output: bool = False,
 ) -> tuple[torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor,
            torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor,
            torch.Tensor, torch.Tensor]:
@@ -908,6 +916,7 @@ def dispatch_mlp_swiglu_combine_bwd_mxfp8(
     Outputs: d_x_shared [T,H], d_x_routed [MB,H], d_gate_shared, d_gate_fp8_routed [MB,I], d_gate_sc_routed, d_up_shared,
              d_up_fp8_routed, d_up_sc_routed, d_hidden_shared, d_hidden_routed [MB,I] bf16, d_y_fp8_routed [MB,H],
              d_y_sc_routed, d_w_shared_gate, d_w_routed_gate, d_w_shared_up, d_w_routed_up, d_w_shared_down, d_w_routed_down
+    (d_x_routed is [0,H] with skip_routed_output: the rows go straight into the owners' slots)
     """
     T, H, I, E = _check_activation_dims(x, w_shared_gate, w_routed_gate)
     _check_layer_scalars(topk, swiglu_limit, num_comm_sms, macrobatch_size, minibatch_size)
@@ -941,7 +950,7 @@ def dispatch_mlp_swiglu_combine_bwd_mxfp8(
                             ("w_shared_down", w_shared_down)))
 
     new = lambda *shape: x.new_empty(shape)  # noqa: E731
-    d_x_shared, d_x_routed, d_hidden_routed = new(T, H), new(MB, H), new(MB, I)
+    d_x_shared, d_x_routed, d_hidden_routed = new(T, H), new(0 if skip_routed_output else MB, H), new(MB, I)
     d_gate_shared, d_up_shared, d_hidden_shared = new(T, I), new(T, I), new(T, I)
     d_gate_q, d_gate_sc = _new_fp8(x, MB, I)
     d_up_q, d_up_sc = _new_fp8(x, MB, I)
