@@ -24,7 +24,6 @@ struct KernelParams {
     const int32_t* tokens_per_expert;
     const int32_t* num_tokens;
     const int32_t* occupied_rows;   // wgrad: see GemmProblem
-    int scale_slots;                // MXFP8: tensor-memory slots the scale columns rotate through
     int num_experts;
     int dense_rows;
     int row_begin, row_end;
@@ -272,7 +271,6 @@ inline KernelParams base_params(const GemmProblem& pb) {
     kp.tokens_per_expert = pb.tokens_per_expert;
     kp.num_tokens = pb.num_tokens;
     kp.occupied_rows = pb.occupied_rows;
-    kp.scale_slots = 1;
     kp.num_experts = pb.num_experts;
     kp.dense_rows = pb.dense_rows;
     kp.row_begin = pb.row_begin;

@@ -20,6 +20,23 @@ int launch_quantize_rows(const void* x, int cols, const int32_t* num_tokens, int
 int launch_dequantize_rows(const void* q, const void* sc, long long sc_row_tile_stride, void* out, int cols,
                            const int32_t* num_tokens, int row_begin, int row_end, cudaStream_t stream);
 
+// Scale byte (biased exponent) of a block whose largest magnitude is `amax`, and the exact reciprocal of the scale.
+__device__ __forceinline__ uint32_t mxfp8_scale_byte(float amax) {
+    const float scale = fmaxf(amax * 0.002232142857f, 0.000000000001f);
+    uint16_t e8m0x2;
+    asm volatile("cvt.rp.satfinite.ue8m0x2.f32 %0, %1, %2;" : "=h"(e8m0x2) : "f"(scale), "f"(scale));
+    return e8m0x2 & 0xFFu;
+}
+__device__ __forceinline__ float mxfp8_inverse_scale(uint32_t scale_byte) { return __uint_as_float((254u - scale_byte) << 23); }
+
+// Four scaled values -> four e4m3 bytes, the first in the low byte.
+__device__ __forceinline__ uint32_t mxfp8_convert4(float a, float b, float c, float d) {
+    uint16_t lo, hi;
+    asm volatile("cvt.rn.satfinite.e4m3x2.f32 %0, %2, %1;" : "=h"(lo) : "f"(a), "f"(b));
+    asm volatile("cvt.rn.satfinite.e4m3x2.f32 %0, %2, %1;" : "=h"(hi) : "f"(c), "f"(d));
+    return static_cast<uint32_t>(lo) | (static_cast<uint32_t>(hi) << 16);
+}
+
 // Quantizes one block of 32 bf16 values (16 packed pairs) to 32 e4m3 bytes (8 words) and one e8m0 scale byte.
 // Same arithmetic as the reference's quantize_single_block (csrc/mxfp8.cuh:45-72).
 __device__ __forceinline__ void mxfp8_quantize_block(const uint32_t (&in)[16], uint32_t (&out)[8], uint32_t& scale_byte) {
@@ -29,19 +46,13 @@ __device__ __forceinline__ void mxfp8_quantize_block(const uint32_t (&in)[16], u
         const float2 f = unpack_bf16x2(in[i]);
         amax = fmaxf(amax, fmaxf(fabsf(f.x), fabsf(f.y)));
     }
-    const float scale = fmaxf(amax * 0.002232142857f, 0.000000000001f);
-    uint16_t e8m0x2;
-    asm volatile("cvt.rp.satfinite.ue8m0x2.f32 %0, %1, %2;" : "=h"(e8m0x2) : "f"(scale), "f"(scale));
-    scale_byte = e8m0x2 & 0xFFu;
-    const float inv = __uint_as_float((254u - scale_byte) << 23);   // 2^(127 - e), exact
+    scale_byte = mxfp8_scale_byte(amax);
+    const float inv = mxfp8_inverse_scale(scale_byte);   // 2^(127 - e), exact
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
         const float2 a = unpack_bf16x2(in[2 * i]);
         const float2 b = unpack_bf16x2(in[2 * i + 1]);
-        uint16_t lo, hi;
-        asm volatile("cvt.rn.satfinite.e4m3x2.f32 %0, %2, %1;" : "=h"(lo) : "f"(a.x * inv), "f"(a.y * inv));
-        asm volatile("cvt.rn.satfinite.e4m3x2.f32 %0, %2, %1;" : "=h"(hi) : "f"(b.x * inv), "f"(b.y * inv));
-        out[i] = static_cast<uint32_t>(lo) | (static_cast<uint32_t>(hi) << 16);
+        out[i] = mxfp8_convert4(a.x * inv, a.y * inv, b.x * inv, b.y * inv);
     }
 }
 
@@ -58,20 +69,14 @@ __device__ __forceinline__ void mxfp8_quantize_quarter(const uint4& in, uint2& o
     }
     amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
     amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
-    const float scale = fmaxf(amax * 0.002232142857f, 0.000000000001f);
-    uint16_t e8m0x2;
-    asm volatile("cvt.rp.satfinite.ue8m0x2.f32 %0, %1, %2;" : "=h"(e8m0x2) : "f"(scale), "f"(scale));
-    scale_byte = e8m0x2 & 0xFFu;
-    const float inv = __uint_as_float((254u - scale_byte) << 23);
+    scale_byte = mxfp8_scale_byte(amax);
+    const float inv = mxfp8_inverse_scale(scale_byte);
     uint32_t o[2];
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
         const float2 a = unpack_bf16x2(w[2 * i]);
         const float2 b = unpack_bf16x2(w[2 * i + 1]);
-        uint16_t lo, hi;
-        asm volatile("cvt.rn.satfinite.e4m3x2.f32 %0, %2, %1;" : "=h"(lo) : "f"(a.x * inv), "f"(a.y * inv));
-        asm volatile("cvt.rn.satfinite.e4m3x2.f32 %0, %2, %1;" : "=h"(hi) : "f"(b.x * inv), "f"(b.y * inv));
-        o[i] = static_cast<uint32_t>(lo) | (static_cast<uint32_t>(hi) << 16);
+        o[i] = mxfp8_convert4(a.x * inv, a.y * inv, b.x * inv, b.y * inv);
     }
     out = make_uint2(o[0], o[1]);
 }

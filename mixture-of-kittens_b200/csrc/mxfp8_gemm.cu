@@ -5,8 +5,12 @@
 // leader CTA issues the MMAs.  In addition every K step carries its e8m0 scales: one 512-byte tile for the CTA's
 // 128 rows of A and two for the 256 columns of B (both CTAs need all B scales), loaded by TMA next to the data,
 // copied to tensor memory with tcgen05.cp and consumed by four K = 32 MMAs whose descriptor selects the scale byte.
-// Tensor memory: 256 accumulator columns + one 12-column scale slot per pipeline stage (16 columns apart), so the
-// accumulator is single-buffered.
+// Tensor memory has no room for two 256-column accumulators beside the scales, so the two that are used share 32
+// columns: the epilogue reads those first and hands them over, and the next tile's MMAs start while the other 224 columns
+// of the finished tile are still being drained.  With one accumulator the tensor pipe stood still for the whole drain
+// (about 1500 clocks per tile of 512 clocks a K step).  Training step before -> after, with the leaner fused epilogue below:
+// hidden 7168, 32 experts of 2048, 16384 tokens 29.4 -> 27.5 ms; hidden 2048, 128 experts of 768, 8192 tokens 4.72 -> 4.00 ms
+// (its gate / up launches 1383 -> 583 us: there the old epilogue was longer than the main loop).
 // Both operands are K-major; the dgrad and wgrad forms use transposed-quantized copies of weights / activations
 // (the role MXFP8 plays in the reference grouped GEMM, csrc/megakernel/grouped_gemm.cuh:222-249).
 #include "gemm_tiles.cuh"
@@ -27,10 +31,15 @@ constexpr int DATA_STAGE_BYTES = A_TILE_BYTES + B_TILE_BYTES;
 constexpr int SCALE_TILE_BYTES = 512;
 constexpr int SCALE_STAGE_BYTES = 3 * SCALE_TILE_BYTES;   // A rows of this CTA, B columns [0,128), B columns [128,256)
 constexpr int STAGE_TX_BYTES = DATA_STAGE_BYTES + SCALE_STAGE_BYTES;
-constexpr int TMEM_SFA_COL = 256;                     // 4 columns
-constexpr int TMEM_SFB_COL = 260;                     // 8 columns
-constexpr int SCALE_SLOT_COLS = 16;                   // columns from one scale slot to the next (slots: up to STAGES)
-
+// Tensor memory (512 columns): two accumulators of 256 columns that share 32 of them, [0, 256) and [224, 480), and two
+// scale slots of 16 columns (4 for A, 8 for B) behind.
+constexpr int ACC_STEP_COLS = 224;
+constexpr int ACC_SHARED_COLS = BN - ACC_STEP_COLS;   // last 32 columns of accumulator 0 = first 32 of accumulator 1
+constexpr int TMEM_SFA_COL = 480;
+constexpr int TMEM_SFB_COL = 484;
+constexpr int SCALE_SLOT_COLS = 16;
+constexpr int SCALE_SLOTS = 2;
+static_assert(TMEM_SFA_COL >= ACC_STEP_COLS + BN && TMEM_SFA_COL + SCALE_SLOTS * SCALE_SLOT_COLS <= TMEM_COLS, "tensor memory");
 
 struct SharedLayout {
     static constexpr int kScales = STAGES * DATA_STAGE_BYTES;
@@ -61,88 +70,83 @@ struct FusedOut {
     float limit;
 };
 
-// One warp = 32 rows of the tile (buffer rows R0 .. R0 + 31, all in one 128-row tile), `packed` = this lane's row:
-// vectors [0, 16) gate, [16, 32) up, already rounded to bf16.
-template <bool CLAMP>
-__device__ __forceinline__ void fused_gate_up_epilogue(const FusedOut& f, const uint4 (&packed)[32], uint8_t* patch, long long R0,
-                                                       int col0, int quarter, int lane) {
-    const long long row_tile = R0 >> 7;
-    const int col_tile = col0 >> 7;
-    const long long sc_off = row_tile * f.sc_row_tile_stride + static_cast<long long>(col_tile) * 512 + lane * 16 + quarter * 4;
-    const long long q_off = R0 * f.cols + col0;
-    // block by block (32 columns), so that the gate / up registers die as the bytes are produced
-    uint4 h[16], gate_bytes[8], up_bytes[8], hid_bytes[8];
-    uint32_t gate_scales = 0, up_scales = 0, hid_scales = 0;
-#pragma unroll
-    for (int b = 0; b < 4; ++b) {
-        uint32_t g[16], u[16], hb[16], out8[8], sbyte;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const uint4 gv = packed[4 * b + i], uv = packed[16 + 4 * b + i];
-            g[4 * i] = gv.x; g[4 * i + 1] = gv.y; g[4 * i + 2] = gv.z; g[4 * i + 3] = gv.w;
-            u[4 * i] = uv.x; u[4 * i + 1] = uv.y; u[4 * i + 2] = uv.z; u[4 * i + 3] = uv.w;
-        }
-#pragma unroll
-        for (int i = 0; i < 16; ++i) hb[i] = swiglu_pair<CLAMP>(g[i], u[i], f.limit);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) h[4 * b + i] = make_uint4(hb[4 * i], hb[4 * i + 1], hb[4 * i + 2], hb[4 * i + 3]);
-        mxfp8_quantize_block(g, out8, sbyte);
-        gate_scales |= sbyte << (8 * b);
-        gate_bytes[2 * b] = make_uint4(out8[0], out8[1], out8[2], out8[3]);
-        gate_bytes[2 * b + 1] = make_uint4(out8[4], out8[5], out8[6], out8[7]);
-        mxfp8_quantize_block(u, out8, sbyte);
-        up_scales |= sbyte << (8 * b);
-        up_bytes[2 * b] = make_uint4(out8[0], out8[1], out8[2], out8[3]);
-        up_bytes[2 * b + 1] = make_uint4(out8[4], out8[5], out8[6], out8[7]);
-        mxfp8_quantize_block(hb, out8, sbyte);
-        hid_scales |= sbyte << (8 * b);
-        hid_bytes[2 * b] = make_uint4(out8[0], out8[1], out8[2], out8[3]);
-        hid_bytes[2 * b + 1] = make_uint4(out8[4], out8[5], out8[6], out8[7]);
-    }
-    *reinterpret_cast<uint32_t*>(f.gate_sc + sc_off) = gate_scales;
-    *reinterpret_cast<uint32_t*>(f.up_sc + sc_off) = up_scales;
-    *reinterpret_cast<uint32_t*>(f.hid_sc + sc_off) = hid_scales;
-    // 128 bytes per row = 64 two-byte elements for the staging helper: full 128-byte lines
-    const long long ld2 = f.cols / 2;
-    epilogue_store_packed_64cols(patch, gate_bytes, reinterpret_cast<bf16*>(f.gate_q + q_off), ld2, lane);
-    epilogue_store_packed_64cols(patch, up_bytes, reinterpret_cast<bf16*>(f.up_q + q_off), ld2, lane);
-    epilogue_store_packed_64cols(patch, hid_bytes, reinterpret_cast<bf16*>(f.hid_q + q_off), ld2, lane);
+// One epilogue warp = 32 rows of the tile (buffer rows R0 .. R0 + 31, all in one 128-row tile), one block of 32 gate
+// columns and the same 32 up columns at a time (`b`, columns col0 + 32 b of the outputs): a lane holds its row of both.
+// The warp's staging patch holds first the three e4m3 outputs of the block (32 bytes per row and output, so that a store
+// instruction fills whole 32-byte sectors), then the bf16 hidden block, which is read back by columns: the warp's 32
+// rows are exactly one scale block of a column, half a warp takes 16 of them for 16 column pairs and the two halves
+// exchange their maxima.  Per block 16 shared-memory words and 2 shuffles a lane, where a butterfly per column over the
+// warp takes 160 shuffles; nothing spills (the whole row in registers took 255 and 0.7 KB of spills).
+constexpr int kBytesPitch = 112;   // 3 x 32 bytes per row; 28 words: conflict free in 16-byte accesses
+constexpr int kHiddenPitch = 80;   // 64 bytes per row; rows >= 16 shifted by 64 bytes: conflict free by rows and columns
+static_assert(32 * kBytesPitch <= kEpiWarpBytes && 32 * kHiddenPitch + 64 <= kEpiWarpBytes, "staging patch too small");
 
-    // transposed layout: for one column the warp's 32 rows are exactly one block of 32; two columns per word
-    uint8_t* sct = f.hid_sct + col_tile * f.sct_row_tile_stride + row_tile * 512 + quarter;
+__device__ __forceinline__ int hidden_offset(int row) { return row * kHiddenPitch + (row >= 16 ? 64 : 0); }
+
+template <bool CLAMP>
+__device__ __forceinline__ void fused_gate_up_block(const FusedOut& f, const uint32_t (&g)[16], const uint32_t (&u)[16], uint8_t* patch,
+                                                    long long R0, int col0, int b, int quarter, int lane, uint32_t (&scales)[3]) {
+    uint32_t h[16];
 #pragma unroll
-    for (int i = 0; i < 16; ++i) {
-        const uint32_t words[4] = {h[i].x, h[i].y, h[i].z, h[i].w};
+    for (int i = 0; i < 16; ++i) h[i] = swiglu_pair<CLAMP>(g[i], u[i], f.limit);
+    uint8_t* mine = patch + lane * kBytesPitch;
+    auto quantize = [&](int o, const uint32_t (&in)[16]) {
+        uint32_t out8[8], sbyte;
+        mxfp8_quantize_block(in, out8, sbyte);
+        scales[o] |= sbyte << (8 * b);
+        *reinterpret_cast<uint4*>(mine + o * 32) = make_uint4(out8[0], out8[1], out8[2], out8[3]);
+        *reinterpret_cast<uint4*>(mine + o * 32 + 16) = make_uint4(out8[4], out8[5], out8[6], out8[7]);
+    };
+    quantize(0, g);
+    quantize(1, u);
+    quantize(2, h);
+    __syncwarp();
+    const long long q_off = R0 * f.cols + col0 + b * 32;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int c = 8 * i + 2 * j;   // columns c, c + 1 of the tile
-            const float2 val = unpack_bf16x2(words[j]);
-            float a0 = fabsf(val.x), a1 = fabsf(val.y);
+    for (int o = 0; o < 3; ++o) {
+        uint8_t* out = (o == 0 ? f.gate_q : o == 1 ? f.up_q : f.hid_q) + q_off;
 #pragma unroll
-            for (int off = 16; off > 0; off >>= 1) {
-                a0 = fmaxf(a0, __shfl_xor_sync(0xffffffffu, a0, off));
-                a1 = fmaxf(a1, __shfl_xor_sync(0xffffffffu, a1, off));
-            }
-            const float s0 = fmaxf(a0 * 0.002232142857f, 0.000000000001f), s1 = fmaxf(a1 * 0.002232142857f, 0.000000000001f);
-            uint16_t e8;
-            asm volatile("cvt.rp.satfinite.ue8m0x2.f32 %0, %1, %2;" : "=h"(e8) : "f"(s1), "f"(s0));   // low byte: s0
-            const uint32_t sb0 = e8 & 0xFFu, sb1 = (e8 >> 8) & 0xFFu;
-            const float inv0 = __uint_as_float((254u - sb0) << 23), inv1 = __uint_as_float((254u - sb1) << 23);
-            uint16_t q2;
-            asm volatile("cvt.rn.satfinite.e4m3x2.f32 %0, %2, %1;" : "=h"(q2) : "f"(val.x * inv0), "f"(val.y * inv1));
-            patch[c * 32 + lane] = static_cast<uint8_t>(q2 & 0xFFu);
-            patch[(c + 1) * 32 + lane] = static_cast<uint8_t>(q2 >> 8);
-            if (lane == (c & 31)) sct[(c & 31) * 16 + (c >> 5) * 4] = static_cast<uint8_t>(sb0);
-            if (lane == ((c + 1) & 31)) sct[((c + 1) & 31) * 16 + ((c + 1) >> 5) * 4] = static_cast<uint8_t>(sb1);
+        for (int it = 0; it < 2; ++it) {
+            const int r = it * 16 + (lane >> 1), seg = (lane & 1) * 16;
+            *reinterpret_cast<uint4*>(out + static_cast<long long>(r) * f.cols + seg) =
+                *reinterpret_cast<const uint4*>(patch + r * kBytesPitch + o * 32 + seg);
         }
     }
     __syncwarp();
-    uint8_t* qt = f.hid_qt + static_cast<long long>(col0) * f.qt_ld + R0;
 #pragma unroll
-    for (int it = 0; it < 8; ++it) {   // 16 columns per store instruction, 32 bytes (the warp's rows) each
-        const int c = it * 16 + (lane >> 1), half = lane & 1;
-        *reinterpret_cast<uint4*>(qt + static_cast<long long>(c) * f.qt_ld + half * 16) =
-            *reinterpret_cast<const uint4*>(patch + c * 32 + half * 16);
+    for (int i = 0; i < 4; ++i)
+        *reinterpret_cast<uint4*>(patch + hidden_offset(lane) + i * 16) = make_uint4(h[4 * i], h[4 * i + 1], h[4 * i + 2], h[4 * i + 3]);
+    __syncwarp();
+    const int pair = lane & 15, half = lane >> 4;   // columns 2 * pair and 2 * pair + 1 of the block, rows [16 * half, +16)
+    uint32_t w[16];
+    float a0 = 0.0f, a1 = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+        w[i] = *reinterpret_cast<const uint32_t*>(patch + hidden_offset(16 * half + i) + pair * 4);
+        const float2 v = unpack_bf16x2(w[i]);
+        a0 = fmaxf(a0, fabsf(v.x));
+        a1 = fmaxf(a1, fabsf(v.y));
+    }
+    a0 = fmaxf(a0, __shfl_xor_sync(0xffffffffu, a0, 16));
+    a1 = fmaxf(a1, __shfl_xor_sync(0xffffffffu, a1, 16));
+    const uint32_t s0 = mxfp8_scale_byte(a0), s1 = mxfp8_scale_byte(a1);
+    const float inv0 = mxfp8_inverse_scale(s0), inv1 = mxfp8_inverse_scale(s1);
+    uint32_t q0[4], q1[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const float2 v0 = unpack_bf16x2(w[4 * i]), v1 = unpack_bf16x2(w[4 * i + 1]), v2 = unpack_bf16x2(w[4 * i + 2]),
+                     v3 = unpack_bf16x2(w[4 * i + 3]);
+        q0[i] = mxfp8_convert4(v0.x * inv0, v1.x * inv0, v2.x * inv0, v3.x * inv0);
+        q1[i] = mxfp8_convert4(v0.y * inv1, v1.y * inv1, v2.y * inv1, v3.y * inv1);
+    }
+    const int c = b * 32 + 2 * pair;
+    uint8_t* qt = f.hid_qt + static_cast<long long>(col0 + c) * f.qt_ld + R0 + half * 16;
+    *reinterpret_cast<uint4*>(qt) = make_uint4(q0[0], q0[1], q0[2], q0[3]);
+    *reinterpret_cast<uint4*>(qt + f.qt_ld) = make_uint4(q1[0], q1[1], q1[2], q1[3]);
+    if (half == 0) {
+        uint8_t* sct = f.hid_sct + (col0 >> 7) * f.sct_row_tile_stride + (R0 >> 7) * 512 + quarter + 2 * pair * 16 + b * 4;
+        sct[0] = static_cast<uint8_t>(s0);
+        sct[16] = static_cast<uint8_t>(s1);
     }
     __syncwarp();
 }
@@ -263,9 +267,11 @@ mxfp8_gemm_kernel(const __grid_constant__ MapSet ms0, const __grid_constant__ Ma
             for (int t = pair; t < num_tiles && ok; t += num_pairs) {
                 Tile tile;
                 if (!decode_tile<MODE, BK>(p, cum, lo, hi, t, tile)) continue;
-                ok = mbar_wait(bar_tmem_empty, (iter & 1u) ^ 1u, abort_flag, p.status);   // epilogue drained the accumulator
+                // the columns that this tile's accumulator shares with the previous one have been read
+                ok = mbar_wait(bar_tmem_empty, (iter & 1u) ^ 1u, abort_flag, p.status);
                 if (!ok) break;
                 tc_fence_after_sync();
+                const uint32_t d_tmem = tmem_base + (iter & 1) * ACC_STEP_COLS;
                 for (int kb = 0; kb < tile.k_blocks; ++kb) {
                     ok = mbar_wait(bar_full + 8 * stage, phase, abort_flag, p.status);
                     if (!ok) break;
@@ -273,8 +279,7 @@ mxfp8_gemm_kernel(const __grid_constant__ MapSet ms0, const __grid_constant__ Ma
                     if (lane == 0) {
                         const uint32_t a_addr = smem_base + stage * DATA_STAGE_BYTES;
                         const uint32_t b_addr = a_addr + A_TILE_BYTES;
-                        // the scale columns rotate with the stage (one slot per stage when scale_slots == STAGES)
-                        const uint32_t slot = static_cast<uint32_t>(stage % p.scale_slots) * SCALE_SLOT_COLS;
+                        const uint32_t slot = static_cast<uint32_t>(stage % SCALE_SLOTS) * SCALE_SLOT_COLS;
                         const uint32_t sfa = sfa_tmem + slot, sfb = sfb_tmem + slot;
                         const uint32_t s_addr = scale_base + stage * SCALE_STAGE_BYTES;
                         tmem_copy_scales_pair(sfa, umma_scale_desc(s_addr));
@@ -284,7 +289,7 @@ mxfp8_gemm_kernel(const __grid_constant__ MapSet ms0, const __grid_constant__ Ma
                         const uint64_t b_desc = umma_smem_desc(b_addr, 16, 1024);
 #pragma unroll
                         for (int k = 0; k < BK / 32; ++k)   // 32 elements = 32 bytes = 2 descriptor units per slice
-                            umma_mxfp8_pair(tmem_base, a_desc + k * 2u, b_desc + k * 2u, umma_idesc_mxfp8(BM, BN, k), sfa, sfb,
+                            umma_mxfp8_pair(d_tmem, a_desc + k * 2u, b_desc + k * 2u, umma_idesc_mxfp8(BM, BN, k), sfa, sfb,
                                             (kb | k) != 0 ? 1u : 0u);
                         umma_commit_pair(bar_empty + 8 * stage);
                         if (kb == tile.k_blocks - 1) umma_commit_pair(bar_tmem_full);
@@ -316,53 +321,66 @@ mxfp8_gemm_kernel(const __grid_constant__ MapSet ms0, const __grid_constant__ Ma
             else
                 out = p.D0 + static_cast<long long>(tile.expert) * p.d_expert_stride +
                       static_cast<long long>(tile.m0 + row_in_tile) * p.ldd + tile.n0;
-            const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
+            const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + (iter & 1) * ACC_STEP_COLS;
             uint8_t* patch = smem_gen + SharedLayout::kEpilogue + quarter * kEpiWarpBytes;
             bf16* warp_out = out - static_cast<long long>(lane) * p.ldd;
-            if (tile.accumulate) {   // rare (later windows of a multi-window backward): add in fp32 per row
-#pragma unroll 1
-                for (int c = 0; c < BN / 32; ++c) {
-                    uint32_t v[32];
-                    tmem_ld_32x32(taddr + c * 32, v);
-                    tmem_ld_wait();
-                    store_row_chunk(out + c * 32, v, true);
-                }
+            // Pieces of the row in an order that starts with the shared columns (the last ones of accumulator 0, the
+            // first ones of accumulator 1); once every warp has them in registers the next tile's MMAs may overwrite them.
+            const int rotate = (iter & 1) ? 0 : 3;
+            auto release_shared_columns = [&]() {
                 tc_fence_before_sync();
                 __syncwarp();
                 if (lane == 0) mbar_arrive_leader(bar_tmem_empty);
-            } else {
-                // The accumulator is single-buffered: read the whole row into registers as packed bf16 first and hand
-                // tensor memory back to the MMA issuer before any of it is written out.
-                uint4 packed[BN / 8];
+            };
+            if (MODE == MODE_ROWS && FUSED) {
+                const long long R0 = tile.row0 - p.row_begin + cta_rank * BM_CTA + quarter * 32;
+                const int col0 = tile.n0 / 2;
+                uint32_t scales[3] = {0, 0, 0};
+#pragma unroll 1
+                for (int j = 0; j < 4; ++j) {
+                    const int b = (j + rotate) & 3;
+                    uint32_t g[16], u[16];
+                    {
+                        uint32_t v0[32], v1[32];
+                        tmem_ld_32x32(taddr + b * 32, v0);
+                        tmem_ld_32x32(taddr + BN_CTA + b * 32, v1);
+                        tmem_ld_wait();
+                        if (j == 0) release_shared_columns();
 #pragma unroll
-                for (int c = 0; c < BN / 64; ++c) {   // two loads in flight per wait
+                        for (int i = 0; i < 16; ++i) {
+                            g[i] = pack_bf16x2(__uint_as_float(v0[2 * i]), __uint_as_float(v0[2 * i + 1]));
+                            u[i] = pack_bf16x2(__uint_as_float(v1[2 * i]), __uint_as_float(v1[2 * i + 1]));
+                        }
+                    }
+                    if (f.clamp) fused_gate_up_block<true>(f, g, u, patch, R0, col0, b, quarter, lane, scales);
+                    else fused_gate_up_block<false>(f, g, u, patch, R0, col0, b, quarter, lane, scales);
+                }
+                const long long sc_off = (R0 >> 7) * f.sc_row_tile_stride + static_cast<long long>(col0 >> 7) * 512 + lane * 16 + quarter * 4;
+                *reinterpret_cast<uint32_t*>(f.gate_sc + sc_off) = scales[0];
+                *reinterpret_cast<uint32_t*>(f.up_sc + sc_off) = scales[1];
+                *reinterpret_cast<uint32_t*>(f.hid_sc + sc_off) = scales[2];
+            } else {
+                bf16* slots[8];
+                if (scattered) spread_slots(slot, slots, lane);
+#pragma unroll 1
+                for (int j = 0; j < BN / 64; ++j) {
+                    const int c = (j + rotate) & 3;
                     uint32_t v0[32], v1[32];
                     tmem_ld_32x32(taddr + c * 64, v0);
                     tmem_ld_32x32(taddr + c * 64 + 32, v1);
                     tmem_ld_wait();
+                    if (j == 0) release_shared_columns();
+                    if (tile.accumulate) {   // rare (later windows of a multi-window backward): add in fp32 per row
+                        store_row_chunk(out + c * 64, v0, true);
+                        store_row_chunk(out + c * 64 + 32, v1, true);
+                    } else if (scattered) {
+                        uint4 packed[8];
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        packed[c * 8 + i] = pack8_bf16(&v0[8 * i]);
-                        packed[c * 8 + 4 + i] = pack8_bf16(&v1[8 * i]);
+                        for (int i = 0; i < 4; ++i) { packed[i] = pack8_bf16(&v0[8 * i]); packed[4 + i] = pack8_bf16(&v1[8 * i]); }
+                        epilogue_scatter_packed_64cols(patch, packed, slots, tile.n0 + c * 64, lane);
+                    } else {
+                        epilogue_store_64cols(patch, v0, v1, warp_out + c * 64, p.ldd, lane);
                     }
-                }
-                tc_fence_before_sync();
-                __syncwarp();
-                if (lane == 0) mbar_arrive_leader(bar_tmem_empty);
-                if (MODE == MODE_ROWS && FUSED) {
-                    const long long R0 = tile.row0 - p.row_begin + cta_rank * BM_CTA + quarter * 32;
-                    if (f.clamp) fused_gate_up_epilogue<true>(f, packed, patch, R0, tile.n0 / 2, quarter, lane);
-                    else fused_gate_up_epilogue<false>(f, packed, patch, R0, tile.n0 / 2, quarter, lane);
-                } else if (scattered) {
-                    bf16* slots[8];
-                    spread_slots(slot, slots, lane);
-#pragma unroll
-                    for (int c = 0; c < BN / 64; ++c)
-                        epilogue_scatter_packed_64cols(patch, &packed[c * 8], slots, tile.n0 + c * 64, lane);
-                } else {
-#pragma unroll
-                    for (int c = 0; c < BN / 64; ++c)
-                        epilogue_store_packed_64cols(patch, &packed[c * 8], warp_out + c * 64, p.ldd, lane);
                 }
             }
             ++iter;
@@ -422,25 +440,11 @@ int fill_set(MapSet* ms, const Fp8Operand& a, long long a_groups, const Fp8Opera
 }
 
 size_t smem_bytes(int num_experts) { return 1024 + SharedLayout::kCum + 4 * (static_cast<size_t>(num_experts) + 2); }
-// Scale slots in tensor memory: one per pipeline stage; MOK_SCALE_SLOTS (1..STAGES) overrides, for measurements.
-int scale_slots() {
-    static int slots = 0;
-    if (slots == 0) {
-        int n = STAGES;
-        if (const char* v = getenv("MOK_SCALE_SLOTS")) {
-            const int want = atoi(v);
-            if (want >= 1 && want <= STAGES) n = want;
-        }
-        slots = n;
-    }
-    return slots;
-}
 
 template <int MODE, bool FUSED = false>
 int launch(const MapSet& ms0, const MapSet& ms1, KernelParams kp, int max_tiles, cudaStream_t stream,
            const FusedOut& fused = FusedOut{}) {
     static int resident_pairs[16] = {0};
-    kp.scale_slots = scale_slots();
     return launch_pairs(mxfp8_gemm_kernel<MODE, FUSED>, "mxfp8_gemm_kernel", resident_pairs, smem_bytes(kp.num_experts), max_tiles,
                         stream, ms0, ms1, kp, fused);
 }
