@@ -60,14 +60,6 @@ __global__ void barrier_kernel(int* local_counter, PeerTable peers, int ep, int*
     asm volatile("fence.acquire.sys;" ::: "memory");
 }
 
-__device__ __forceinline__ uint32_t scale_pair(uint32_t v, float w) {
-    const float2 f = unpack_bf16x2(v);
-    return pack_bf16x2(f.x * w, f.y * w);
-}
-__device__ __forceinline__ uint4 scale_vec(uint4 a, float w) {
-    return make_uint4(scale_pair(a.x, w), scale_pair(a.y, w), scale_pair(a.z, w), scale_pair(a.w, w));
-}
-
 // ---- staging of de-duplicated tokens -----------------------------------------------------------------------
 // One warp per staged token of the range first used by rows [from_row, min(to_row, *num_tokens)).
 __global__ void __launch_bounds__(256) stage_tokens_kernel(PeerTable src, const int* __restrict__ unique_peer,

@@ -132,8 +132,9 @@ bool overlap_enabled() {
 // minibatch_size sets the hand-over granularity (the default 4096 gives 32768-row chunks, the size that measured best
 // on the DeepSeek-V3-shaped layer).  MOK_CHUNK_ROWS overrides the row count (rounded up to whole minibatches).
 // A window is cut into equal chunks of about that size; one that holds less than one and a half of them stays whole.
-int chunk_rows_for(const mok_layer_args* a, int window_rows) {
-    long long rows = static_cast<long long>(kMinibatchesPerChunk) * a->minibatch_size;
+// Without anything to hand over (`whole`) it stays whole too: every further launch adds a nearly empty last wave of tiles.
+int chunk_rows_for(const mok_layer_args* a, int window_rows, bool whole) {
+    long long rows = whole ? window_rows : static_cast<long long>(kMinibatchesPerChunk) * a->minibatch_size;
     if (const char* v = getenv("MOK_CHUNK_ROWS")) {
         const int r = atoi(v);
         if (r > 0) rows = r;
@@ -445,10 +446,38 @@ int quantize_span(const mok_layer_args* a, const Span& s, const void* src, int c
                                 qt_, a->macrobatch_size, sct_, scale_tile_row_bytes(a->macrobatch_size), st);
 }
 
-// x (bf16, dispatched) -> x_fp8 (+ transpose) -> gate, up (bf16 scratch + saved e4m3) -> hidden (bf16 scratch, e4m3 + transpose)
+// One rank, MXFP8: the quantizer reads the tokens of its rows itself (and scales them by `weights`), so that no dispatch
+// pass writes the rows as bf16 for it to read back (4 of 8 bytes per element).  Several ranks keep the dispatch, which
+// overlaps its NVLink transfers with the GEMMs.
+bool gathers_in_quantizer(const mok_layer_args* a) { return a->ep_size == 1; }
+
+int quantize_local_rows(const mok_layer_args* a, const Span& s, const uint64_t* src_ptrs, const uint64_t* weight_ptrs,
+                        float* row_weight, void* q, void* sc, void* qt, void* sct, cudaStream_t st) {
+    const int H = a->hidden;
+    const long long off = s.begin - s.base, scH = scale_tile_row_bytes(H);
+    LocalRows g{};
+    g.rows = rows_of(a, s);
+    g.topk = a->topk;
+    g.num_routes = a->num_local_tokens * a->topk;
+    if (weight_ptrs != nullptr) {
+        if (weight_ptrs[0] == 0) return MOK_ERR_INVALID_ARGUMENT;
+        g.weights = reinterpret_cast<const float*>(weight_ptrs[0]);
+        g.row_weight = at_row(row_weight, s, 1);
+    }
+    return launch_quantize_rows(reinterpret_cast<const void*>(src_ptrs[0]), H, a->num_tokens, s.begin, s.end,
+                                static_cast<uint8_t*>(q) + off * H, static_cast<uint8_t*>(sc) + (off / 128) * scH, scH,
+                                static_cast<uint8_t*>(qt) + off, a->macrobatch_size, static_cast<uint8_t*>(sct) + (off / 128) * 512,
+                                scale_tile_row_bytes(a->macrobatch_size), st, &g);
+}
+
+// x (bf16: dispatched, or read by the quantizer) -> x_fp8 (+ transpose) -> gate, up (bf16 scratch + saved e4m3) -> hidden
+// (bf16 scratch, e4m3 + transpose)
 int gate_up_hidden_mxfp8(const mok_layer_args* a, const Span& s, cudaStream_t st) {
     const int H = a->hidden, I = a->intermediate;
-    MOK_TRY(quantize_span(a, s, a->x_routed, H, a->x_fp8, a->x_sc, a->x_fp8_t, a->x_sc_t, st));
+    if (gathers_in_quantizer(a))
+        MOK_TRY(quantize_local_rows(a, s, a->x_ptrs, nullptr, nullptr, a->x_fp8, a->x_sc, a->x_fp8_t, a->x_sc_t, st));
+    else
+        MOK_TRY(quantize_span(a, s, a->x_routed, H, a->x_fp8, a->x_sc, a->x_fp8_t, a->x_sc_t, st));
     const Fp8Operand wg = weight_operand(a, a->w_gate_fp8, a->w_gate_sc, I, H);
     const Fp8Operand wu = weight_operand(a, a->w_up_fp8, a->w_up_sc, I, H);
     if (fused_activations_enabled() && fused_epilogue_enabled()) {   // SwiGLU and the quantizations in the GEMM epilogue
@@ -507,8 +536,8 @@ int check_mxfp8_forward_fields(const mok_layer_args* a) {
 // On return every pull has been consumed; pushes may still be running on the internal stream (the caller joins).
 template <class Pull, class Compute, class Push>
 int run_chunks(const mok_layer_args* a, const Span& win, bool overlapped, DeviceStreams* d, cudaStream_t main_stream,
-               Pull pull, Compute compute, Push push) {
-    const int chunk = chunk_rows_for(a, win.end - win.begin);
+               Pull pull, Compute compute, Push push, bool whole = false) {
+    const int chunk = chunk_rows_for(a, win.end - win.begin, whole);
     const int n = (win.end - win.begin + chunk - 1) / chunk;
     auto span_of = [&](int c) {
         Span s;
@@ -705,7 +734,9 @@ extern "C" int mok_moe_forward_mxfp8(const mok_layer_args* a, mok_stream_t strea
     if (a->w_shared_gate && (!a->w_shared_down || !a->y_shared)) return MOK_ERR_INVALID_ARGUMENT;
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
     Staging x_staging, d_y_staging;   // how far the de-duplicated tokens of x / d_y have been staged in this call
-    const bool overlapped = overlap_enabled();
+    const bool gather = gathers_in_quantizer(a);
+    const bool local = gather && a->y_routed == nullptr;   // nothing to pull, nothing to push: one stream, whole windows
+    const bool overlapped = overlap_enabled() && !local;
     DeviceStreams* d = nullptr;
     CommFork fork;
     if (overlapped) MOK_TRY(fork.start(s, &d));
@@ -720,7 +751,9 @@ extern "C" int mok_moe_forward_mxfp8(const mok_layer_args* a, mok_stream_t strea
         const Span win = window_span(a, wi);
         MOK_TRY(run_chunks(
             a, win, overlapped, d, s,
-            [&](const Span& c, int ctas, cudaStream_t st) { return dispatch_x(a, c, ctas, st, &x_staging); },
+            [&](const Span& c, int ctas, cudaStream_t st) {
+                return gather ? static_cast<int>(MOK_OK) : dispatch_x(a, c, ctas, st, &x_staging);
+            },
             [&](const Span& c, cudaStream_t st) {
                 MOK_TRY(gate_up_hidden_mxfp8(a, c, st));
                 RowScatter slots;
@@ -732,7 +765,8 @@ extern "C" int mok_moe_forward_mxfp8(const mok_layer_args* a, mok_stream_t strea
                 if (a->y_routed == nullptr) return static_cast<int>(MOK_OK);
                 return launch_combine(a->combine_ptrs, nullptr, a->ep_size, rows_of(a, c), a->topk, a->num_local_tokens, H,
                                       rows_bf16(a->y_routed, c, H), nullptr, ctas, st);
-            }));
+            },
+            local));
         if (overlapped) {
             MOK_TRY(order_after(d, d->comm, s));
             if (wi > 0) MOK_TRY(order_after(d, s, d->comm));
@@ -749,7 +783,7 @@ extern "C" int mok_moe_recompute_mxfp8(const mok_layer_args* a, mok_stream_t str
     Staging x_staging, d_y_staging;   // how far the de-duplicated tokens of x / d_y have been staged in this call
     if (a->w_shared_gate) MOK_TRY(shared_up_to_hidden(a, s));
     const Span win = window_span(a, 0);
-    MOK_TRY(dispatch_x(a, win, 0, s, &x_staging));
+    if (!gathers_in_quantizer(a)) MOK_TRY(dispatch_x(a, win, 0, s, &x_staging));
     MOK_TRY(gate_up_hidden_mxfp8(a, win, s));
     return MOK_OK;
 }
@@ -775,7 +809,9 @@ extern "C" int mok_moe_backward_mxfp8(const mok_layer_args* a, mok_stream_t stre
     Staging x_staging, d_y_staging;   // how far the de-duplicated tokens of x / d_y have been staged in this call
     const int H = a->hidden, I = a->intermediate, T = a->num_local_tokens;
     const bool clamp = a->has_swiglu_limit != 0;
-    const bool overlapped = overlap_enabled();
+    const bool gather = gathers_in_quantizer(a);
+    const bool local = gather && a->d_x_routed == nullptr;   // nothing to pull, nothing to push: one stream, whole windows
+    const bool overlapped = overlap_enabled() && !local;
     DeviceStreams* d = nullptr;
     CommFork fork;
     if (overlapped) MOK_TRY(fork.start(s, &d));
@@ -797,19 +833,25 @@ extern "C" int mok_moe_backward_mxfp8(const mok_layer_args* a, mok_stream_t stre
     for (int wi = 0; wi < num_windows(a); ++wi) {
         const Span win = window_span(a, wi);
         if (wi > 0) {
-            MOK_TRY(dispatch_x(a, win, 0, s, &x_staging));
+            if (!gather) MOK_TRY(dispatch_x(a, win, 0, s, &x_staging));
             MOK_TRY(gate_up_hidden_mxfp8(a, win, s));
         }
         MOK_TRY(run_chunks(
             a, win, overlapped, d, s,
-            [&](const Span& c, int ctas, cudaStream_t st) { return dispatch_d_y(a, c, row_weight, ctas, st, &d_y_staging); },
+            [&](const Span& c, int ctas, cudaStream_t st) {
+                return gather ? static_cast<int>(MOK_OK) : dispatch_d_y(a, c, row_weight, ctas, st, &d_y_staging);
+            },
             [&](const Span& c, cudaStream_t st) {
                 const GemmProblem p = routed_problem(a, c);
                 const long long off = c.begin - c.base;
                 RowScatter slots;
                 if (a->d_x_routed == nullptr)
                     MOK_TRY(slots_of(a, a->d_x_routed_ptrs, a->d_router_weight_ptrs, at_row(row_grad, c, 1), &slots));
-                MOK_TRY(quantize_span(a, c, a->d_y_routed, H, a->d_y_fp8, a->d_y_sc, a->d_y_fp8_t, a->d_y_sc_t, st));
+                if (gather)
+                    MOK_TRY(quantize_local_rows(a, c, a->d_y_ptrs, a->router_weight_ptrs, row_weight, a->d_y_fp8, a->d_y_sc,
+                                                a->d_y_fp8_t, a->d_y_sc_t, st));
+                else
+                    MOK_TRY(quantize_span(a, c, a->d_y_routed, H, a->d_y_fp8, a->d_y_sc, a->d_y_fp8_t, a->d_y_sc_t, st));
                 MOK_TRY(launch_fp8_rows_gemm(p, act_rows(a, a->d_y_fp8, a->d_y_sc, H, c), H, wd_t, nullptr,
                                              rows_bf16(a->d_hidden_routed, c, I), nullptr, I, st));
                 if (fused_activations_enabled()) {   // saved e4m3 gate / up + d_hidden -> e4m3 d_gate, d_up in one pass
@@ -850,7 +892,8 @@ extern "C" int mok_moe_backward_mxfp8(const mok_layer_args* a, mok_stream_t stre
                 if (a->d_x_routed == nullptr) return static_cast<int>(MOK_OK);
                 return launch_combine(a->d_x_routed_ptrs, a->d_router_weight_ptrs, a->ep_size, rows_of(a, c), a->topk, T, H,
                                       rows_bf16(a->d_x_routed, c, H), at_row(row_grad, c, 1), ctas, st);
-            }));
+            },
+            local));
         GemmProblem p = routed_problem(a, win);
         if (wgrad_trim_enabled()) p.occupied_rows = occupied;
         MOK_TRY(launch_fp8_wgrad_gemm(p, act_transposed(a, a->d_y_fp8_t, a->d_y_sc_t, H), H,

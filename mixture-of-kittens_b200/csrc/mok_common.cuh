@@ -57,6 +57,14 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
 __device__ __forceinline__ float2 unpack_bf16x2(uint32_t v) {
     return __bfloat1622float2(*reinterpret_cast<__nv_bfloat162*>(&v));
 }
+// eight bf16 values times w, rounded to bf16
+__device__ __forceinline__ uint32_t scale_pair(uint32_t v, float w) {
+    const float2 f = unpack_bf16x2(v);
+    return pack_bf16x2(f.x * w, f.y * w);
+}
+__device__ __forceinline__ uint4 scale_vec(uint4 a, float w) {
+    return make_uint4(scale_pair(a.x, w), scale_pair(a.y, w), scale_pair(a.z, w), scale_pair(a.w, w));
+}
 
 // ---------------------------------------------------------------------------------------------
 // mbarrier

@@ -21,8 +21,6 @@ constexpr int kRowPitch = kTile * 2 + 16;   // bytes; the 16-byte pad keeps row-
 constexpr int kOutPitch = kTile + 16;       // bytes per staged e4m3 output row
 constexpr int kQuantSmemBytes = kTile * (kRowPitch + kOutPitch);
 
-int enable_quantize_smem();   // raises the kernel's dynamic shared-memory limit once per device
-
 // 128 rows x 128 bytes from the staging tile to global memory, eight lanes per row: every store instruction of a
 // warp writes four complete 128-byte lines (a thread writing its own row would touch 32 lines with 16 bytes each).
 __device__ __forceinline__ void store_staged_rows(const uint8_t* otile, uint8_t* out, long long ld, int tid) {
@@ -90,21 +88,53 @@ struct QuantArgs {
     int row_begin, row_end;    // schedule rows covered by the span (row_end also bounds a dense matrix)
 };
 
-__global__ void __launch_bounds__(128) quantize_kernel(const QuantArgs a) {
+// GATHER: the tile's rows are schedule rows whose tokens are read where they lie (`x` = all tokens of this rank), and
+// with weights scaled on the way, instead of from a buffer that a dispatch pass has filled.
+template <bool GATHER>
+__global__ void __launch_bounds__(128) quantize_kernel(const QuantArgs a, const LocalRows g) {
     extern __shared__ __align__(16) uint8_t quant_smem[];
     uint8_t* tile = quant_smem;                                  // bf16 input tile, padded rows
     uint8_t* otile = quant_smem + kTile * kRowPitch;             // e4m3 rows staged for full-line stores
     const int tid = threadIdx.x;
     const int tc = blockIdx.x, tr = blockIdx.y, e = blockIdx.z;
+    if (GATHER && tc == 0 && tr == 0 && tid == 0 && *a.num_tokens > g.rows.covered_rows && g.rows.status != nullptr)
+        atomicOr(g.rows.status, (uint32_t)MOK_STATUS_BAD_SCHEDULE_ENTRY);
     const int limit = a.num_tokens != nullptr ? min(a.row_end, *a.num_tokens) : a.row_end;
     if (a.row_begin + tr * kTile >= limit) return;
-    const bf16* src = a.x + e * a.x_mat_stride + static_cast<long long>(tr) * kTile * a.x_ld + static_cast<long long>(tc) * kTile;
 
+    if (GATHER) {
+        int* tokens = reinterpret_cast<int*>(otile);             // both free until the first store_staged_rows
+        float* scales = reinterpret_cast<float*>(otile) + kTile;
+        const int row = a.row_begin + tr * kTile + tid;
+        const int peer = g.rows.peer_rank[row], route = g.rows.peer_token[row];
+        const bool valid = peer == 0 && route >= 0 && route < g.num_routes;
+        if (peer >= 0 && !valid && tc == 0 && g.rows.status != nullptr)
+            atomicOr(g.rows.status, (uint32_t)MOK_STATUS_BAD_SCHEDULE_ENTRY);
+        const float w = valid && g.weights != nullptr ? g.weights[route] : 0.0f;
+        tokens[tid] = valid ? route / g.topk : -1;
+        scales[tid] = w;
+        if (tc == 0 && g.weights != nullptr) g.row_weight[tr * kTile + tid] = w;
+        __syncthreads();
+        const bf16* src = a.x + static_cast<long long>(tc) * kTile + (tid & 15) * 8;
+#pragma unroll 8
+        for (int j = 0; j < 16; ++j) {
+            const int r = (tid >> 4) + 8 * j;
+            const int token = tokens[r];
+            uint4 val = make_uint4(0, 0, 0, 0);                  // padding row: zeros, as a dispatch writes them
+            if (token >= 0) {
+                val = *reinterpret_cast<const uint4*>(src + token * a.x_ld);
+                if (g.weights != nullptr) val = scale_vec(val, scales[r]);
+            }
+            *reinterpret_cast<uint4*>(tile + r * kRowPitch + (tid & 15) * 16) = val;
+        }
+    } else {
+        const bf16* src = a.x + e * a.x_mat_stride + static_cast<long long>(tr) * kTile * a.x_ld + static_cast<long long>(tc) * kTile;
 #pragma unroll 4
-    for (int i = tid; i < kTile * 16; i += 128) {   // 128 rows x 16 vectors of 16 bytes, coalesced along the row
-        const int r = i >> 4, v = i & 15;
-        const uint4 val = *reinterpret_cast<const uint4*>(src + static_cast<long long>(r) * a.x_ld + v * 8);
-        *reinterpret_cast<uint4*>(tile + r * kRowPitch + v * 16) = val;
+        for (int i = tid; i < kTile * 16; i += 128) {   // 128 rows x 16 vectors of 16 bytes, coalesced along the row
+            const int r = i >> 4, v = i & 15;
+            const uint4 val = *reinterpret_cast<const uint4*>(src + static_cast<long long>(r) * a.x_ld + v * 8);
+            *reinterpret_cast<uint4*>(tile + r * kRowPitch + v * 16) = val;
+        }
     }
     __syncthreads();
 
@@ -302,15 +332,25 @@ __global__ void __launch_bounds__(256) dequantize_kernel(const uint8_t* __restri
     }
 }
 
-int enable_quantize_smem() {
-    static bool done[16] = {false};
+// Raises the dynamic shared-memory limit of one kernel instantiation once per device.
+template <typename Kernel>
+int enable_tile_smem(Kernel kernel, bool (&done)[16]) {
     int dev = 0;
     MOK_CUDA_CHECK(cudaGetDevice(&dev));
     if (dev < 0 || dev >= 16) return MOK_ERR_UNSUPPORTED;
     if (!done[dev]) {
-        MOK_CUDA_CHECK(cudaFuncSetAttribute(quantize_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kQuantSmemBytes));
+        MOK_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kQuantSmemBytes));
         done[dev] = true;
     }
+    return MOK_OK;
+}
+
+template <bool GATHER>
+int launch_quantize(const QuantArgs& a, const LocalRows& g, const dim3& grid, cudaStream_t stream) {
+    static bool done[16] = {false};
+    if (int rc = enable_tile_smem(quantize_kernel<GATHER>, done)) return rc;
+    quantize_kernel<GATHER><<<grid, 128, kQuantSmemBytes, stream>>>(a, g);
+    MOK_LAUNCH_CHECK("mxfp8_quantize_kernel");
     return MOK_OK;
 }
 
@@ -318,10 +358,13 @@ int enable_quantize_smem() {
 
 int launch_quantize_rows(const void* x, int cols, const int32_t* num_tokens, int row_begin, int row_end, void* q, void* sc,
                          long long sc_row_tile_stride, void* qt, long long qt_ld, void* sct, long long sct_row_tile_stride,
-                         cudaStream_t stream) {
+                         cudaStream_t stream, const LocalRows* gather) {
     if (x == nullptr || cols <= 0 || cols % 128 != 0 || row_end <= row_begin || (row_end - row_begin) % 128 != 0)
         return MOK_ERR_INVALID_ARGUMENT;
     if ((q == nullptr) != (sc == nullptr) || (qt == nullptr) != (sct == nullptr) || (q == nullptr && qt == nullptr))
+        return MOK_ERR_INVALID_ARGUMENT;
+    if (gather != nullptr && ((reinterpret_cast<uintptr_t>(x) & 15u) != 0 || num_tokens == nullptr || !gather->rows.peer_rank ||
+                              !gather->rows.peer_token || gather->topk < 1 || (gather->weights != nullptr && !gather->row_weight)))
         return MOK_ERR_INVALID_ARGUMENT;
     QuantArgs a{};
     a.x = static_cast<const bf16*>(x);
@@ -339,10 +382,7 @@ int launch_quantize_rows(const void* x, int cols, const int32_t* num_tokens, int
     const int row_tiles = (row_end - row_begin) / 128;
     if (row_tiles > 65535) return MOK_ERR_TOO_LARGE;
     dim3 grid(cols / 128, row_tiles, 1);
-    if (int rc = enable_quantize_smem()) return rc;
-    quantize_kernel<<<grid, 128, kQuantSmemBytes, stream>>>(a);
-    MOK_LAUNCH_CHECK("mxfp8_quantize_kernel");
-    return MOK_OK;
+    return gather != nullptr ? launch_quantize<true>(a, *gather, grid, stream) : launch_quantize<false>(a, LocalRows{}, grid, stream);
 }
 
 int launch_dequantize_rows(const void* q, const void* sc, long long sc_row_tile_stride, void* out, int cols,
@@ -361,19 +401,6 @@ int launch_dequantize_rows(const void* q, const void* sc, long long sc_row_tile_
 }
 
 namespace {
-
-// Raises the dynamic shared-memory limit of one kernel instantiation once per device.
-template <typename Kernel>
-int enable_tile_smem(Kernel kernel, bool (&done)[16]) {
-    int dev = 0;
-    MOK_CUDA_CHECK(cudaGetDevice(&dev));
-    if (dev < 0 || dev >= 16) return MOK_ERR_UNSUPPORTED;
-    if (!done[dev]) {
-        MOK_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kQuantSmemBytes));
-        done[dev] = true;
-    }
-    return MOK_OK;
-}
 
 template <typename Kernel, typename Args>
 int launch_tile_kernel(Kernel kernel, const char* name, bool (&done)[16], const Args& args, int cols, int rows, cudaStream_t stream) {
@@ -503,8 +530,5 @@ extern "C" int mok_mxfp8_quantize(const void* x_bf16, int num_matrices, int rows
     a.row_begin = 0;
     a.row_end = rows;
     dim3 grid(cols / 128, rows / 128, num_matrices);
-    if (int rc = enable_quantize_smem()) return rc;
-    quantize_kernel<<<grid, 128, kQuantSmemBytes, reinterpret_cast<cudaStream_t>(stream)>>>(a);
-    MOK_LAUNCH_CHECK("mxfp8_quantize_kernel");
-    return MOK_OK;
+    return launch_quantize<false>(a, LocalRows{}, grid, reinterpret_cast<cudaStream_t>(stream));
 }

@@ -4,17 +4,28 @@
 #include <cuda_fp16.h>
 #include <cuda_fp8.h>
 
-#include "mok_common.cuh"
+#include "comm.cuh"
 
 namespace mok {
+
+// Schedule rows whose tokens lie in this rank's own memory.  With `weights` (fp32 per route) every row is multiplied by
+// its weight (rounded to bf16), which is also written to row_weight[row - rows.row_begin] (0 on padding rows).
+struct LocalRows {
+    RowWindow rows;
+    int topk, num_routes;
+    const float* weights;
+    float* row_weight;
+};
 
 // Quantizes schedule rows [row_begin, min(row_end, *num_tokens)) of a bf16 activation buffer whose row 0 (`x`) holds
 // schedule row row_begin.  Normal output: q (same shape) + scale tiles at sc + row_tile * sc_row_tile_stride +
 // col_tile * 512.  Transposed output: element (c, r) at qt[c * qt_ld + r] (qt points at the column of row_begin) +
 // scale tiles at sct + col_tile * sct_row_tile_stride + row_tile * 512.  Either pair may be nullptr.
+// With `gather` the rows are not in a buffer yet: `x` is this rank's [num_local_tokens, cols] input and every schedule row
+// is read from its token (rows of one rank only; padding rows are zeros), scaled and reported like launch_dispatch does.
 int launch_quantize_rows(const void* x, int cols, const int32_t* num_tokens, int row_begin, int row_end, void* q, void* sc,
                          long long sc_row_tile_stride, void* qt, long long qt_ld, void* sct, long long sct_row_tile_stride,
-                         cudaStream_t stream);
+                         cudaStream_t stream, const LocalRows* gather = nullptr);
 
 // bf16 out[r, c] = value of the MXFP8 element (exact), same row window convention.
 int launch_dequantize_rows(const void* q, const void* sc, long long sc_row_tile_stride, void* out, int cols,
