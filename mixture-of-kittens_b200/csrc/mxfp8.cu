@@ -18,58 +18,77 @@ namespace {
 
 constexpr int kTile = 128;
 constexpr int kRowPitch = kTile * 2 + 16;   // bytes; the 16-byte pad keeps row-wise 16 B reads conflict free
-constexpr int kOutPitch = kTile + 16;       // bytes per staged e4m3 output row
-constexpr int kQuantSmemBytes = kTile * (kRowPitch + kOutPitch);
+constexpr int kOutPitch = kTile + 16;       // bytes per staged e4m3 output row; staged over the bf16 tile it came from
+constexpr int kTileBytes = kTile * kRowPitch;
 
 // 128 rows x 128 bytes from the staging tile to global memory, eight lanes per row: every store instruction of a
 // warp writes four complete 128-byte lines (a thread writing its own row would touch 32 lines with 16 bytes each).
+template <int THREADS>
 __device__ __forceinline__ void store_staged_rows(const uint8_t* otile, uint8_t* out, long long ld, int tid) {
-#pragma unroll 4
-    for (int i = tid; i < kTile * 8; i += 128) {
+#pragma unroll
+    for (int i = tid; i < kTile * 8; i += THREADS) {
         const int r = i >> 3, seg = i & 7;
         *reinterpret_cast<uint4*>(out + static_cast<long long>(r) * ld + seg * 16) =
             *reinterpret_cast<const uint4*>(otile + r * kOutPitch + seg * 16);
     }
 }
 
-// Transposed layout of a staged bf16 tile: thread = column of the tile = row of the transpose, four blocks of 32 down
-// the column.  `out` is the transposed tile's first byte (rows `ld` apart), `scale_tile` its 512-byte scale tile.
-// Every thread of the block calls; the tile must be complete (a barrier before the call is the caller's).
-// A thread takes two adjacent columns (one 32-bit shared-memory word per row, conflict free across the warp) and two of
-// the four row blocks: threads 0..63 the blocks 0 and 1, threads 64..127 the blocks 2 and 3.
-__device__ __forceinline__ void quantize_tile_transposed(const uint8_t* tile, uint8_t* otile, int tid, uint8_t* out, long long ld,
-                                                         uint8_t* scale_tile) {
-    const int pair = tid & 63, half = tid >> 6;
+// One 512-byte scale tile from shared memory: single scale bytes stored to global memory would be a quarter of all store
+// requests of a tile.
+constexpr int kScaleTile = 512;
+__device__ __forceinline__ void store_scale_tile(const uint8_t* staged, uint8_t* out, int tid) {
+    if (tid < kScaleTile / 16) reinterpret_cast<uint4*>(out)[tid] = reinterpret_cast<const uint4*>(staged)[tid];
+}
+
+// Transposed layout of a staged bf16 tile: column of the tile = row of the transpose, four blocks of 32 down the column.
+// `out` is the transposed tile's first byte (rows `ld` apart), `scale_tile` its 512-byte scale tile.  THREADS threads (128 or
+// 256) with tid 0.. take one tile; every thread of the block calls, and the tile must be complete (a barrier before the call
+// is the caller's).  A thread takes two adjacent columns (one 32-bit shared-memory word per row, conflict free across the
+// warp) and one or two of the four row blocks.  The e4m3 rows and the scale bytes are staged over the tile itself, which
+// nobody reads any more by then, and leave as full lines.
+template <int THREADS>
+__device__ __forceinline__ void quantize_tile_transposed(uint8_t* tile, int tid, uint8_t* out, long long ld, uint8_t* scale_tile) {
+    constexpr int kBlocks = 256 / THREADS;
+    const int pair = tid & 63, first = (tid >> 6) * kBlocks;
     const int col_a = 2 * pair, col_b = col_a + 1;
-    uint32_t scales_a = 0, scales_b = 0;
+    uint32_t sa[kBlocks], sb[kBlocks];
+    uint32_t qa[kBlocks][8], qb[kBlocks][8];
 #pragma unroll
-    for (int k = 0; k < 2; ++k) {
-        const int kb = 2 * half + k;
-        uint32_t pa[16], pb[16];
+    for (int k = 0; k < kBlocks; ++k) {
+        const uint8_t* column = tile + (first + k) * 32 * kRowPitch + pair * 4;
+        uint32_t w[32], m = 0;
 #pragma unroll
-        for (int i = 0; i < 16; ++i) {
-            const uint32_t w0 = *reinterpret_cast<const uint32_t*>(tile + (kb * 32 + 2 * i) * kRowPitch + pair * 4);
-            const uint32_t w1 = *reinterpret_cast<const uint32_t*>(tile + (kb * 32 + 2 * i + 1) * kRowPitch + pair * 4);
-            pa[i] = __byte_perm(w0, w1, 0x5410);   // low halves: column a of rows 2i, 2i + 1
-            pb[i] = __byte_perm(w0, w1, 0x7632);   // high halves: column b
+        for (int i = 0; i < 32; ++i) w[i] = *reinterpret_cast<const uint32_t*>(column + i * kRowPitch);
+#pragma unroll
+        for (int i = 0; i < 32; ++i) m = bf16x2_absmax(m, w[i]);
+        const float2 amax = unpack_bf16x2(m);
+        sa[k] = mxfp8_scale_byte(amax.x);
+        sb[k] = mxfp8_scale_byte(amax.y);
+        const float inv_a = mxfp8_inverse_scale(sa[k]), inv_b = mxfp8_inverse_scale(sb[k]);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const float2 v0 = unpack_bf16x2(w[4 * i]), v1 = unpack_bf16x2(w[4 * i + 1]), v2 = unpack_bf16x2(w[4 * i + 2]),
+                         v3 = unpack_bf16x2(w[4 * i + 3]);
+            qa[k][i] = mxfp8_convert4(v0.x * inv_a, v1.x * inv_a, v2.x * inv_a, v3.x * inv_a);
+            qb[k][i] = mxfp8_convert4(v0.y * inv_b, v1.y * inv_b, v2.y * inv_b, v3.y * inv_b);
         }
-        uint32_t out8[8], sbyte;
-        mxfp8_quantize_block(pa, out8, sbyte);
-        scales_a |= sbyte << (k * 8);
-        uint8_t* dst = otile + col_a * kOutPitch + kb * 32;
-        *reinterpret_cast<uint4*>(dst) = make_uint4(out8[0], out8[1], out8[2], out8[3]);
-        *reinterpret_cast<uint4*>(dst + 16) = make_uint4(out8[4], out8[5], out8[6], out8[7]);
-        mxfp8_quantize_block(pb, out8, sbyte);
-        scales_b |= sbyte << (k * 8);
-        dst = otile + col_b * kOutPitch + kb * 32;
-        *reinterpret_cast<uint4*>(dst) = make_uint4(out8[0], out8[1], out8[2], out8[3]);
-        *reinterpret_cast<uint4*>(dst + 16) = make_uint4(out8[4], out8[5], out8[6], out8[7]);
     }
     __syncthreads();
-    store_staged_rows(otile, out, ld, tid);
-    // scale bytes of row blocks 2 * half and 2 * half + 1 of the transposed rows col_a and col_b
-    *reinterpret_cast<uint16_t*>(scale_tile + (col_a & 31) * 16 + (col_a >> 5) * 4 + 2 * half) = static_cast<uint16_t>(scales_a);
-    *reinterpret_cast<uint16_t*>(scale_tile + (col_b & 31) * 16 + (col_b >> 5) * 4 + 2 * half) = static_cast<uint16_t>(scales_b);
+    uint8_t* staged_scales = tile + kTile * kOutPitch;
+#pragma unroll
+    for (int k = 0; k < kBlocks; ++k) {
+        uint4* dst_a = reinterpret_cast<uint4*>(tile + col_a * kOutPitch + (first + k) * 32);
+        uint4* dst_b = reinterpret_cast<uint4*>(tile + col_b * kOutPitch + (first + k) * 32);
+        dst_a[0] = make_uint4(qa[k][0], qa[k][1], qa[k][2], qa[k][3]);
+        dst_a[1] = make_uint4(qa[k][4], qa[k][5], qa[k][6], qa[k][7]);
+        dst_b[0] = make_uint4(qb[k][0], qb[k][1], qb[k][2], qb[k][3]);
+        dst_b[1] = make_uint4(qb[k][4], qb[k][5], qb[k][6], qb[k][7]);
+        staged_scales[(col_a & 31) * 16 + (col_a >> 5) * 4 + first + k] = static_cast<uint8_t>(sa[k]);
+        staged_scales[(col_b & 31) * 16 + (col_b >> 5) * 4 + first + k] = static_cast<uint8_t>(sb[k]);
+    }
+    __syncthreads();
+    store_staged_rows<THREADS>(tile, out, ld, tid);
+    store_scale_tile(staged_scales, scale_tile, tid);
 }
 
 struct QuantArgs {
@@ -88,84 +107,101 @@ struct QuantArgs {
     int row_begin, row_end;    // schedule rows covered by the span (row_end also bounds a dense matrix)
 };
 
+__device__ __forceinline__ void copy_async_16(void* dst, const void* src, bool valid) {   // zeros when not valid
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(valid ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void copy_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int PENDING>
+__device__ __forceinline__ void copy_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(PENDING) : "memory"); }
+
+// Bound by HBM.  A block walks `tiles_per_block` column tiles of one row tile; the next tile is on its way into the second
+// buffer while one is being quantized.  One tile per block and plain loads left the block waiting for its own loads two
+// thirds of the time, whatever the order of the tiles: 37k gathered rows of 7168 359 us (242 us with the leaner arithmetic
+// and 6 instead of 4 resident blocks), now 197 us (5.5 TB/s); weights 32 x 2048 x 7168 441 -> 419 us.  16 lanes per row and eight consecutive columns per lane, eight rows per thread: a block of 32 along the row is four adjacent lanes,
+// so the normal layout is quantized from registers (mxfp8_quantize_quarter) and stored as full 128-byte lines.
 // GATHER: the tile's rows are schedule rows whose tokens are read where they lie (`x` = all tokens of this rank), and
 // with weights scaled on the way, instead of from a buffer that a dispatch pass has filled.
+constexpr int kQuantThreads = 256;
+constexpr int kQuantBlocksPerSm = 3;
 template <bool GATHER>
-__global__ void __launch_bounds__(128) quantize_kernel(const QuantArgs a, const LocalRows g) {
-    extern __shared__ __align__(16) uint8_t quant_smem[];
-    uint8_t* tile = quant_smem;                                  // bf16 input tile, padded rows
-    uint8_t* otile = quant_smem + kTile * kRowPitch;             // e4m3 rows staged for full-line stores
-    const int tid = threadIdx.x;
-    const int tc = blockIdx.x, tr = blockIdx.y, e = blockIdx.z;
-    if (GATHER && tc == 0 && tr == 0 && tid == 0 && *a.num_tokens > g.rows.covered_rows && g.rows.status != nullptr)
+__global__ void __launch_bounds__(kQuantThreads, kQuantBlocksPerSm) quantize_kernel(const QuantArgs a, const LocalRows g, int tiles_per_block) {
+    extern __shared__ __align__(16) uint8_t quant_tiles[];       // two bf16 input tiles, padded rows
+    __shared__ __align__(16) uint8_t row_scales[kScaleTile];
+    __shared__ int tokens[GATHER ? kTile : 1];
+    __shared__ float scales[GATHER ? kTile : 1];
+    const int tid = threadIdx.x, v = tid & 15, rq = tid >> 4;
+    const int tc0 = blockIdx.x * tiles_per_block, tr = blockIdx.y, e = blockIdx.z;
+    if (GATHER && tc0 == 0 && tr == 0 && tid == 0 && *a.num_tokens > g.rows.covered_rows && g.rows.status != nullptr)
         atomicOr(g.rows.status, (uint32_t)MOK_STATUS_BAD_SCHEDULE_ENTRY);
     const int limit = a.num_tokens != nullptr ? min(a.row_end, *a.num_tokens) : a.row_end;
     if (a.row_begin + tr * kTile >= limit) return;
 
+    const bf16* src = a.x + static_cast<long long>(tc0) * kTile + v * 8;
     if (GATHER) {
-        int* tokens = reinterpret_cast<int*>(otile);             // both free until the first store_staged_rows
-        float* scales = reinterpret_cast<float*>(otile) + kTile;
-        const int row = a.row_begin + tr * kTile + tid;
-        const int peer = g.rows.peer_rank[row], route = g.rows.peer_token[row];
-        const bool valid = peer == 0 && route >= 0 && route < g.num_routes;
-        if (peer >= 0 && !valid && tc == 0 && g.rows.status != nullptr)
-            atomicOr(g.rows.status, (uint32_t)MOK_STATUS_BAD_SCHEDULE_ENTRY);
-        const float w = valid && g.weights != nullptr ? g.weights[route] : 0.0f;
-        tokens[tid] = valid ? route / g.topk : -1;
-        scales[tid] = w;
-        if (tc == 0 && g.weights != nullptr) g.row_weight[tr * kTile + tid] = w;
-        __syncthreads();
-        const bf16* src = a.x + static_cast<long long>(tc) * kTile + (tid & 15) * 8;
-#pragma unroll 8
-        for (int j = 0; j < 16; ++j) {
-            const int r = (tid >> 4) + 8 * j;
-            const int token = tokens[r];
-            uint4 val = make_uint4(0, 0, 0, 0);                  // padding row: zeros, as a dispatch writes them
-            if (token >= 0) {
-                val = *reinterpret_cast<const uint4*>(src + token * a.x_ld);
-                if (g.weights != nullptr) val = scale_vec(val, scales[r]);
-            }
-            *reinterpret_cast<uint4*>(tile + r * kRowPitch + (tid & 15) * 16) = val;
+        if (tid < kTile) {
+            const int row = a.row_begin + tr * kTile + tid;
+            const int peer = g.rows.peer_rank[row], route = g.rows.peer_token[row];
+            const bool valid = peer == 0 && route >= 0 && route < g.num_routes;
+            if (peer >= 0 && !valid && tc0 == 0 && g.rows.status != nullptr)
+                atomicOr(g.rows.status, (uint32_t)MOK_STATUS_BAD_SCHEDULE_ENTRY);
+            const float w = valid && g.weights != nullptr ? g.weights[route] : 0.0f;
+            tokens[tid] = valid ? route / g.topk : -1;
+            scales[tid] = w;
+            if (tc0 == 0 && g.weights != nullptr) g.row_weight[tr * kTile + tid] = w;
         }
+        __syncthreads();
     } else {
-        const bf16* src = a.x + e * a.x_mat_stride + static_cast<long long>(tr) * kTile * a.x_ld + static_cast<long long>(tc) * kTile;
-#pragma unroll 4
-        for (int i = tid; i < kTile * 16; i += 128) {   // 128 rows x 16 vectors of 16 bytes, coalesced along the row
-            const int r = i >> 4, v = i & 15;
-            const uint4 val = *reinterpret_cast<const uint4*>(src + static_cast<long long>(r) * a.x_ld + v * 8);
-            *reinterpret_cast<uint4*>(tile + r * kRowPitch + v * 16) = val;
-        }
+        src += e * a.x_mat_stride + static_cast<long long>(tr) * kTile * a.x_ld;
     }
-    __syncthreads();
-
-    if (a.q != nullptr) {   // thread = row of the tile, four blocks of 32 along the row
-        uint32_t scale_word = 0;
-        uint8_t* out = a.q + e * a.q_mat_stride + static_cast<long long>(tr) * kTile * a.x_ld + static_cast<long long>(tc) * kTile;
-        uint8_t* mine = otile + tid * kOutPitch;
+    const int tiles = min(tiles_per_block, static_cast<int>(a.x_ld / kTile) - tc0);
+    auto fetch = [&](int t) {
+        uint8_t* dst = quant_tiles + (t & 1) * kTileBytes + v * 16;
 #pragma unroll
-        for (int kb = 0; kb < 4; ++kb) {
-            uint32_t packed[16];
+        for (int j = 0; j < 8; ++j) {
+            const int r = rq + 16 * j;
+            const int token = GATHER ? tokens[r] : r;            // padding row: zeros, as a dispatch writes them
+            copy_async_16(dst + r * kRowPitch, src + t * kTile + max(token, 0) * a.x_ld, token >= 0);
+        }
+        copy_async_commit();
+    };
+    fetch(0);
+    for (int t = 0; t < tiles; ++t) {
+        if (t + 1 < tiles) {
+            fetch(t + 1);
+            copy_async_wait<1>();
+        } else {
+            copy_async_wait<0>();
+        }
+        const int tc = tc0 + t;
+        uint8_t* tile = quant_tiles + (t & 1) * kTileBytes;
+        uint8_t* q = a.q + e * a.q_mat_stride + static_cast<long long>(tr) * kTile * a.x_ld + static_cast<long long>(tc) * kTile + v * 8;
 #pragma unroll
-            for (int v = 0; v < 4; ++v) {
-                const uint4 val = *reinterpret_cast<const uint4*>(tile + tid * kRowPitch + kb * 64 + v * 16);
-                packed[v * 4 + 0] = val.x; packed[v * 4 + 1] = val.y; packed[v * 4 + 2] = val.z; packed[v * 4 + 3] = val.w;
+        for (int j = 0; j < 8; ++j) {                            // the rows that this thread has fetched itself
+            const int r = rq + 16 * j;
+            uint4* mine = reinterpret_cast<uint4*>(tile + r * kRowPitch + v * 16);
+            uint4 val = *mine;
+            if (GATHER && g.weights != nullptr && tokens[r] >= 0) {
+                val = scale_vec(val, scales[r]);
+                *mine = val;
             }
-            uint32_t out8[8], sbyte;
-            mxfp8_quantize_block(packed, out8, sbyte);
-            scale_word |= sbyte << (kb * 8);
-            *reinterpret_cast<uint4*>(mine + kb * 32) = make_uint4(out8[0], out8[1], out8[2], out8[3]);
-            *reinterpret_cast<uint4*>(mine + kb * 32 + 16) = make_uint4(out8[4], out8[5], out8[6], out8[7]);
+            if (a.q != nullptr) {
+                uint2 bytes;
+                uint32_t sb;
+                mxfp8_quantize_quarter(val, bytes, sb);
+                *reinterpret_cast<uint2*>(q + r * a.x_ld) = bytes;
+                if ((v & 3) == 0) row_scales[(r & 31) * 16 + (r >> 5) * 4 + (v >> 2)] = static_cast<uint8_t>(sb);
+            }
         }
         __syncthreads();
-        store_staged_rows(otile, out, a.x_ld, tid);
-        __syncthreads();
-        uint8_t* sdst = a.sc + e * a.sc_mat_stride + tr * a.sc_row_tile_stride + static_cast<long long>(tc) * 512;
-        *reinterpret_cast<uint32_t*>(sdst + (tid & 31) * 16 + (tid >> 5) * 4) = scale_word;
+        if (a.q != nullptr)
+            store_scale_tile(row_scales, a.sc + e * a.sc_mat_stride + tr * a.sc_row_tile_stride + static_cast<long long>(tc) * kScaleTile, tid);
+        if (a.qt != nullptr)
+            quantize_tile_transposed<kQuantThreads>(
+                tile, tid,
+                a.qt + e * a.qt_mat_stride + static_cast<long long>(tc) * kTile * a.qt_ld + static_cast<long long>(tr) * kTile,
+                a.qt_ld, a.sct + e * a.sct_mat_stride + tc * a.sct_row_tile_stride + static_cast<long long>(tr) * kScaleTile);
+        if (t + 1 < tiles) __syncthreads();                      // the tile and the scale bytes may be overwritten
     }
-    if (a.qt != nullptr)
-        quantize_tile_transposed(tile, otile, tid,
-                                 a.qt + e * a.qt_mat_stride + static_cast<long long>(tc) * kTile * a.qt_ld + static_cast<long long>(tr) * kTile,
-                                 a.qt_ld, a.sct + e * a.sct_mat_stride + tc * a.sct_row_tile_stride + static_cast<long long>(tr) * 512);
 }
 
 // ---- fused activation steps ---------------------------------------------------------------------------------------
@@ -184,9 +220,7 @@ struct FusedFwdArgs {
 
 template <bool CLAMP>
 __global__ void __launch_bounds__(128) swiglu_quantize_fwd_kernel(const FusedFwdArgs a) {
-    extern __shared__ __align__(16) uint8_t quant_smem[];
-    uint8_t* tile = quant_smem;
-    uint8_t* otile = quant_smem + kTile * kRowPitch;
+    __shared__ __align__(16) uint8_t tile[kTileBytes];
     const int tid = threadIdx.x, v = tid & 15, rq = tid >> 4;
     const int tc = blockIdx.x, tr = blockIdx.y;
     const int limit_row = min(a.row_end, *a.num_tokens);
@@ -218,7 +252,7 @@ __global__ void __launch_bounds__(128) swiglu_quantize_fwd_kernel(const FusedFwd
         *reinterpret_cast<uint4*>(tile + r * kRowPitch + v * 16) = h;
     }
     __syncthreads();
-    quantize_tile_transposed(tile, otile, tid, a.hidden_qt + static_cast<long long>(tc) * kTile * a.qt_ld + static_cast<long long>(tr) * kTile,
+    quantize_tile_transposed<128>(tile, tid, a.hidden_qt + static_cast<long long>(tc) * kTile * a.qt_ld + static_cast<long long>(tr) * kTile,
                              a.qt_ld, a.hidden_sct + tc * a.sct_row_tile_stride + static_cast<long long>(tr) * 512);
 }
 
@@ -233,57 +267,69 @@ struct FusedBwdArgs {
     float limit;
 };
 
+// 256 threads, 8 rows each; d_gate and d_up have a tile of their own, and half of the block transposes each.  135k rows of
+// 2048: 997 us with one tile (d_up waited in 64 registers, 16 warps per SM, loads in the order of use), 720 us like this.
 template <bool CLAMP>
-__global__ void __launch_bounds__(128) swiglu_quantize_bwd_kernel(const FusedBwdArgs a) {
-    extern __shared__ __align__(16) uint8_t quant_smem[];
-    uint8_t* tile = quant_smem;
-    uint8_t* otile = quant_smem + kTile * kRowPitch;
+__global__ void __launch_bounds__(256, 3) swiglu_quantize_bwd_kernel(const FusedBwdArgs a) {
+    extern __shared__ __align__(16) uint8_t bwd_tiles[];
+    __shared__ __align__(16) uint8_t row_scales[2][kScaleTile];
     const int tid = threadIdx.x, v = tid & 15, rq = tid >> 4;
     const int tc = blockIdx.x, tr = blockIdx.y;
     const int limit_row = min(a.row_end, *a.num_tokens);
     if (a.row_begin + tr * kTile >= limit_row) return;
     const long long sc_off = tr * a.sc_row_tile_stride + static_cast<long long>(tc) * 512;
     const int tiles = a.cols / kTile;
-    uint4 du_keep[16];   // d_up waits in registers while d_gate uses the shared-memory tile
+#pragma unroll 1
+    for (int part = 0; part < 2; ++part) {
+        uint2 gq[4], uq[4];   // four rows in flight before the first of them is used
+        uint4 dh[4];
+        uint32_t gs[4], us[4];
 #pragma unroll
-    for (int j = 0; j < 16; ++j) {
-        const int r = rq + 8 * j;
-        const long long row = static_cast<long long>(tr) * kTile + r;
-        const long long off = row * a.cols + tc * kTile + v * 8;
-        const uint2 gq = *reinterpret_cast<const uint2*>(a.gate_q + off);
-        const uint2 uq = *reinterpret_cast<const uint2*>(a.up_q + off);
-        const uint4 dh = *reinterpret_cast<const uint4*>(a.d_hidden + off);
-        const int sidx = (r & 31) * 16 + (r >> 5) * 4 + (v >> 2);
-        const uint4 g = mxfp8_dequantize8(gq, a.gate_sc[sc_off + sidx]);
-        const uint4 u = mxfp8_dequantize8(uq, a.up_sc[sc_off + sidx]);
-        uint4 dg, du;
-        float acc = swiglu_bwd_pair<CLAMP>(g.x, u.x, dh.x, a.limit, dg.x, du.x);
-        acc += swiglu_bwd_pair<CLAMP>(g.y, u.y, dh.y, a.limit, dg.y, du.y);
-        acc += swiglu_bwd_pair<CLAMP>(g.z, u.z, dh.z, a.limit, dg.z, du.z);
-        acc += swiglu_bwd_pair<CLAMP>(g.w, u.w, dh.w, a.limit, dg.w, du.w);
+        for (int j = 0; j < 4; ++j) {
+            const int r = rq + 16 * (4 * part + j);
+            const long long off = (static_cast<long long>(tr) * kTile + r) * a.cols + tc * kTile + v * 8;
+            const int sidx = (r & 31) * 16 + (r >> 5) * 4 + (v >> 2);
+            gq[j] = __ldg(reinterpret_cast<const uint2*>(a.gate_q + off));
+            uq[j] = __ldg(reinterpret_cast<const uint2*>(a.up_q + off));
+            dh[j] = __ldg(reinterpret_cast<const uint4*>(a.d_hidden + off));
+            gs[j] = __ldg(a.gate_sc + sc_off + sidx);
+            us[j] = __ldg(a.up_sc + sc_off + sidx);
+        }
 #pragma unroll
-        for (int off_l = 1; off_l < 16; off_l <<= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off_l);   // the row's 16 lanes
-        if (v == 0) a.row_partial[row * tiles + tc] = acc;
-        uint2 q;
-        uint32_t sb;
-        mxfp8_quantize_quarter(dg, q, sb);
-        *reinterpret_cast<uint2*>(a.dg_q + off) = q;
-        if ((v & 3) == 0) a.dg_sc[sc_off + sidx] = static_cast<uint8_t>(sb);
-        mxfp8_quantize_quarter(du, q, sb);
-        *reinterpret_cast<uint2*>(a.du_q + off) = q;
-        if ((v & 3) == 0) a.du_sc[sc_off + sidx] = static_cast<uint8_t>(sb);
-        *reinterpret_cast<uint4*>(tile + r * kRowPitch + v * 16) = dg;
-        du_keep[j] = du;
+        for (int j = 0; j < 4; ++j) {
+            const int r = rq + 16 * (4 * part + j);
+            const long long row = static_cast<long long>(tr) * kTile + r;
+            const long long off = row * a.cols + tc * kTile + v * 8;
+            const int sidx = (r & 31) * 16 + (r >> 5) * 4 + (v >> 2);
+            const uint4 g = mxfp8_dequantize8(gq[j], gs[j]);
+            const uint4 u = mxfp8_dequantize8(uq[j], us[j]);
+            uint4 dg, du;
+            float acc = swiglu_bwd_pair<CLAMP>(g.x, u.x, dh[j].x, a.limit, dg.x, du.x);
+            acc += swiglu_bwd_pair<CLAMP>(g.y, u.y, dh[j].y, a.limit, dg.y, du.y);
+            acc += swiglu_bwd_pair<CLAMP>(g.z, u.z, dh[j].z, a.limit, dg.z, du.z);
+            acc += swiglu_bwd_pair<CLAMP>(g.w, u.w, dh[j].w, a.limit, dg.w, du.w);
+#pragma unroll
+            for (int off_l = 1; off_l < 16; off_l <<= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off_l);   // the row's 16 lanes
+            if (v == 0) a.row_partial[row * tiles + tc] = acc;
+            uint2 q;
+            uint32_t sb;
+            mxfp8_quantize_quarter(dg, q, sb);
+            *reinterpret_cast<uint2*>(a.dg_q + off) = q;
+            if ((v & 3) == 0) row_scales[0][sidx] = static_cast<uint8_t>(sb);
+            mxfp8_quantize_quarter(du, q, sb);
+            *reinterpret_cast<uint2*>(a.du_q + off) = q;
+            if ((v & 3) == 0) row_scales[1][sidx] = static_cast<uint8_t>(sb);
+            *reinterpret_cast<uint4*>(bwd_tiles + r * kRowPitch + v * 16) = dg;
+            *reinterpret_cast<uint4*>(bwd_tiles + kTileBytes + r * kRowPitch + v * 16) = du;
+        }
     }
     __syncthreads();
     const long long t_off = static_cast<long long>(tc) * kTile * a.qt_ld + static_cast<long long>(tr) * kTile;
     const long long ts_off = tc * a.sct_row_tile_stride + static_cast<long long>(tr) * 512;
-    quantize_tile_transposed(tile, otile, tid, a.dg_qt + t_off, a.qt_ld, a.dg_sct + ts_off);
-    __syncthreads();
-#pragma unroll
-    for (int j = 0; j < 16; ++j) *reinterpret_cast<uint4*>(tile + (rq + 8 * j) * kRowPitch + v * 16) = du_keep[j];
-    __syncthreads();
-    quantize_tile_transposed(tile, otile, tid, a.du_qt + t_off, a.qt_ld, a.du_sct + ts_off);
+    const bool up = tid >= 128;
+    store_scale_tile(row_scales[up], (up ? a.du_sc : a.dg_sc) + sc_off, tid & 127);
+    quantize_tile_transposed<128>(bwd_tiles + (up ? kTileBytes : 0), tid & 127, (up ? a.du_qt : a.dg_qt) + t_off, a.qt_ld,
+                             (up ? a.du_sct : a.dg_sct) + ts_off);
 }
 
 __global__ void __launch_bounds__(256) router_grad_kernel(const float* __restrict__ row_partial, int tiles,
@@ -332,24 +378,22 @@ __global__ void __launch_bounds__(256) dequantize_kernel(const uint8_t* __restri
     }
 }
 
-// Raises the dynamic shared-memory limit of one kernel instantiation once per device.
-template <typename Kernel>
-int enable_tile_smem(Kernel kernel, bool (&done)[16]) {
+template <bool GATHER>
+int launch_quantize(const QuantArgs& a, const LocalRows& g, const dim3& tiles, cudaStream_t stream) {
+    static bool done[16] = {false};
     int dev = 0;
     MOK_CUDA_CHECK(cudaGetDevice(&dev));
     if (dev < 0 || dev >= 16) return MOK_ERR_UNSUPPORTED;
     if (!done[dev]) {
-        MOK_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kQuantSmemBytes));
+        MOK_CUDA_CHECK(cudaFuncSetAttribute(quantize_kernel<GATHER>, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * kTileBytes));
         done[dev] = true;
     }
-    return MOK_OK;
-}
-
-template <bool GATHER>
-int launch_quantize(const QuantArgs& a, const LocalRows& g, const dim3& grid, cudaStream_t stream) {
-    static bool done[16] = {false};
-    if (int rc = enable_tile_smem(quantize_kernel<GATHER>, done)) return rc;
-    quantize_kernel<GATHER><<<grid, 128, kQuantSmemBytes, stream>>>(a, g);
+    // as many tiles per block as leave every resident block at least two turns, up to 8
+    const long long total = static_cast<long long>(tiles.x) * tiles.y * tiles.z;
+    long long per_block = total / (2LL * kQuantBlocksPerSm * sm_count());
+    per_block = per_block < 1 ? 1 : per_block > 8 ? 8 : per_block;
+    const dim3 grid((tiles.x + per_block - 1) / per_block, tiles.y, tiles.z);
+    quantize_kernel<GATHER><<<grid, kQuantThreads, 2 * kTileBytes, stream>>>(a, g, static_cast<int>(per_block));
     MOK_LAUNCH_CHECK("mxfp8_quantize_kernel");
     return MOK_OK;
 }
@@ -402,12 +446,20 @@ int launch_dequantize_rows(const void* q, const void* sc, long long sc_row_tile_
 
 namespace {
 
+// `smem`: dynamic shared memory, whose limit is raised once per device and kernel instantiation.
 template <typename Kernel, typename Args>
-int launch_tile_kernel(Kernel kernel, const char* name, bool (&done)[16], const Args& args, int cols, int rows, cudaStream_t stream) {
+int launch_tile_kernel(Kernel kernel, const char* name, bool (&done)[16], const Args& args, int cols, int rows, int threads, int smem,
+                       cudaStream_t stream) {
     if (rows / 128 > 65535) return MOK_ERR_TOO_LARGE;
-    if (int rc = enable_tile_smem(kernel, done)) return rc;
+    int dev = 0;
+    MOK_CUDA_CHECK(cudaGetDevice(&dev));
+    if (dev < 0 || dev >= 16) return MOK_ERR_UNSUPPORTED;
+    if (smem > 0 && !done[dev]) {
+        MOK_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        done[dev] = true;
+    }
     dim3 grid(cols / 128, rows / 128, 1);
-    kernel<<<grid, 128, kQuantSmemBytes, stream>>>(args);
+    kernel<<<grid, threads, smem, stream>>>(args);
     MOK_LAUNCH_CHECK(name);
     return MOK_OK;
 }
@@ -443,9 +495,9 @@ int launch_swiglu_quantize_fwd(const void* gate, const void* up, int cols, const
     static bool done_clamp[16] = {false}, done_plain[16] = {false};
     if (has_limit)
         return launch_tile_kernel(swiglu_quantize_fwd_kernel<true>, "swiglu_quantize_fwd_kernel", done_clamp, a, cols,
-                                  row_end - row_begin, stream);
+                                  row_end - row_begin, 128, 0, stream);
     return launch_tile_kernel(swiglu_quantize_fwd_kernel<false>, "swiglu_quantize_fwd_kernel", done_plain, a, cols,
-                              row_end - row_begin, stream);
+                              row_end - row_begin, 128, 0, stream);
 }
 
 int launch_swiglu_quantize_bwd(const void* gate_q, const void* gate_sc, const void* up_q, const void* up_sc, const void* d_hidden,
@@ -483,9 +535,9 @@ int launch_swiglu_quantize_bwd(const void* gate_q, const void* gate_sc, const vo
     static bool done_clamp[16] = {false}, done_plain[16] = {false};
     if (has_limit)
         return launch_tile_kernel(swiglu_quantize_bwd_kernel<true>, "swiglu_quantize_bwd_kernel", done_clamp, a, cols,
-                                  row_end - row_begin, stream);
+                                  row_end - row_begin, 256, 2 * kTileBytes, stream);
     return launch_tile_kernel(swiglu_quantize_bwd_kernel<false>, "swiglu_quantize_bwd_kernel", done_plain, a, cols,
-                              row_end - row_begin, stream);
+                              row_end - row_begin, 256, 2 * kTileBytes, stream);
 }
 
 int launch_router_grad(const float* row_partial, int tiles, const float* row_weight, float* row_grad, const int32_t* num_tokens,

@@ -31,6 +31,12 @@ int launch_quantize_rows(const void* x, int cols, const int32_t* num_tokens, int
 int launch_dequantize_rows(const void* q, const void* sc, long long sc_row_tile_stride, void* out, int cols,
                            const int32_t* num_tokens, int row_begin, int row_end, cudaStream_t stream);
 
+// max(m, |v|) of both bf16 halves: exact, and like fmaxf it passes over NaNs, at half an instruction per element.
+__device__ __forceinline__ uint32_t bf16x2_absmax(uint32_t m, uint32_t v) {
+    const __nv_bfloat162 r = __hmax2(*reinterpret_cast<const __nv_bfloat162*>(&m), __habs2(*reinterpret_cast<const __nv_bfloat162*>(&v)));
+    return *reinterpret_cast<const uint32_t*>(&r);
+}
+
 // Scale byte (biased exponent) of a block whose largest magnitude is `amax`, and the exact reciprocal of the scale.
 __device__ __forceinline__ uint32_t mxfp8_scale_byte(float amax) {
     const float scale = fmaxf(amax * 0.002232142857f, 0.000000000001f);
@@ -51,13 +57,11 @@ __device__ __forceinline__ uint32_t mxfp8_convert4(float a, float b, float c, fl
 // Quantizes one block of 32 bf16 values (16 packed pairs) to 32 e4m3 bytes (8 words) and one e8m0 scale byte.
 // Same arithmetic as the reference's quantize_single_block (csrc/mxfp8.cuh:45-72).
 __device__ __forceinline__ void mxfp8_quantize_block(const uint32_t (&in)[16], uint32_t (&out)[8], uint32_t& scale_byte) {
-    float amax = 0.0f;
+    uint32_t m = 0;
 #pragma unroll
-    for (int i = 0; i < 16; ++i) {
-        const float2 f = unpack_bf16x2(in[i]);
-        amax = fmaxf(amax, fmaxf(fabsf(f.x), fabsf(f.y)));
-    }
-    scale_byte = mxfp8_scale_byte(amax);
+    for (int i = 0; i < 16; ++i) m = bf16x2_absmax(m, in[i]);
+    const float2 amax = unpack_bf16x2(m);
+    scale_byte = mxfp8_scale_byte(fmaxf(amax.x, amax.y));
     const float inv = mxfp8_inverse_scale(scale_byte);   // 2^(127 - e), exact
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
@@ -72,15 +76,13 @@ __device__ __forceinline__ void mxfp8_quantize_block(const uint32_t (&in)[16], u
 // Bit-identical to mxfp8_quantize_block.  All four lanes receive the scale byte.
 __device__ __forceinline__ void mxfp8_quantize_quarter(const uint4& in, uint2& out, uint32_t& scale_byte) {
     const uint32_t w[4] = {in.x, in.y, in.z, in.w};
-    float amax = 0.0f;
+    uint32_t m = 0;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const float2 f = unpack_bf16x2(w[i]);
-        amax = fmaxf(amax, fmaxf(fabsf(f.x), fabsf(f.y)));
-    }
-    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
-    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
-    scale_byte = mxfp8_scale_byte(amax);
+    for (int i = 0; i < 4; ++i) m = bf16x2_absmax(m, w[i]);
+    m = bf16x2_absmax(m, __shfl_xor_sync(0xffffffffu, m, 1));
+    m = bf16x2_absmax(m, __shfl_xor_sync(0xffffffffu, m, 2));
+    const float2 amax = unpack_bf16x2(m);
+    scale_byte = mxfp8_scale_byte(fmaxf(amax.x, amax.y));
     const float inv = mxfp8_inverse_scale(scale_byte);
     uint32_t o[2];
 #pragma unroll
