@@ -263,6 +263,8 @@ def _scatter_from_gemm(workspace: MoKWorkspace) -> bool:
 
 
 def _barrier(workspace: MoKWorkspace) -> None:
+    if workspace.ep_size == 1:
+        return   # nobody to wait for: stream order is enough, and five dispatcher round trips a training step are not free
     barrier_all(workspace.barrier_buffer, workspace.barrier_buffer_ptrs, workspace.barrier_buffer_multicast_ptr,
                 workspace.barrier_target)
 
