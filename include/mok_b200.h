@@ -268,6 +268,10 @@ typedef struct mok_layer_args {
     void *staged_x, *staged_d_y;
     int staged_rows;
     int reserved1;
+    /* Optional scratch of the bf16 calls, used when the experts hold few rows each (NULL: padding rows are computed too). */
+    int32_t* occupied_rows;   /* forward, recompute: int32 [num_local_experts] (the backward has room for this in row_scratch) */
+    float* row_partials;      /* backward: fp32 [MB * intermediate / 128]; the SwiGLU backward then runs in the epilogue of the
+                                 down projection's input gradient */
 } mok_layer_args;
 
 /*

@@ -23,7 +23,7 @@ struct KernelParams {
     RowScatter scatter;             // rows forms: output rows go to their owners' slots instead of D0 (see grouped_gemm.cuh)
     const int32_t* tokens_per_expert;
     const int32_t* num_tokens;
-    const int32_t* occupied_rows;   // wgrad: see GemmProblem
+    const int32_t* occupied_rows;   // see GemmProblem
     int num_experts;
     int dense_rows;
     int row_begin, row_end;
@@ -37,7 +37,10 @@ struct KernelParams {
     bf16* D0;
     bf16* D1;
     bf16* D2;                 // bf16 kernel, fused gate / up form: hidden = silu(gate) * up (D0 = gate, D1 = up)
-    int clamp;                // fused gate / up form: SwiGLU clamp on
+    const bf16* gate;         // routed bf16 kernel, SwiGLU backward: saved gate / up (D0 = d_hidden or nullptr, D1 = d_gate, D2 = d_up)
+    const bf16* up;
+    float* row_partial;       // and per row and 128 columns the sum of d_hidden * hidden, [rows, N / 128], or nullptr
+    int clamp;                // fused SwiGLU forms: clamp on
     float limit;
     int out_f32;              // bf16 kernel: D0 is an fp32 array (router logits and router weight gradient)
     long long ldd;
@@ -292,7 +295,7 @@ inline int rows_group(long long expert_weight_bytes) { return expert_weight_byte
 
 // Launches `kernel` as clusters of two CTAs, as many pairs as can be resident at once (at most one per tile).
 // `resident_pairs` caches the occupancy query per device and kernel instantiation.
-template <typename Kernel, typename... Args>
+template <int THREADS = NUM_THREADS, typename Kernel, typename... Args>
 int launch_pairs(Kernel kernel, const char* name, int (&resident_pairs)[16], size_t smem, int max_tiles, cudaStream_t stream,
                  const Args&... args) {
     int dev = 0;
@@ -304,7 +307,7 @@ int launch_pairs(Kernel kernel, const char* name, int (&resident_pairs)[16], siz
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
     cudaLaunchConfig_t cfg = {};
-    cfg.blockDim = dim3(NUM_THREADS);
+    cfg.blockDim = dim3(THREADS);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
     cfg.attrs = attr;

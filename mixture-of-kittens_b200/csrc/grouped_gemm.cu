@@ -346,12 +346,22 @@ int launch(const CUtensorMap& a0, const CUtensorMap& b0, const CUtensorMap& a1, 
 
 }  // namespace
 
+// routed_gemm.cu: the rows forms for problems that know their occupied rows (arguments already checked)
+int launch_routed_gemm(const GemmProblem& pb, const void* A0, const void* A1, int K, const void* B0, const void* B1, void* D, int N,
+                       bool b_is_kn, cudaStream_t stream, const RowScatter* scatter);
+int launch_routed_gate_up(const GemmProblem& pb, const void* A, int K, const void* Wg, const void* Wu, void* gate, void* up, void* hidden,
+                          int N, bool has_limit, float limit, cudaStream_t stream);
+int launch_routed_down_dgrad(const GemmProblem& pb, const void* A, int K, const void* B, const void* gate, const void* up, void* d_hidden,
+                             void* d_gate, void* d_up, float* row_partial, int N, bool has_limit, float limit, cudaStream_t stream);
+
 int launch_rows_gemm(const GemmProblem& pb, const void* A, int K, const void* B0, const void* B1, void* D0, void* D1,
                      int N, bool b_is_kn, cudaStream_t stream, const RowScatter* scatter) {
     int rc = check_problem(pb);
     if (rc != MOK_OK) return rc;
     if (K <= 0 || N <= 0 || K % BK != 0 || N % BN != 0) return MOK_ERR_INVALID_ARGUMENT;
     const int n_sets = (B1 != nullptr) ? 2 : 1;
+    if (pb.occupied_rows != nullptr && n_sets == 1)
+        return launch_routed_gemm(pb, A, nullptr, K, B0, nullptr, D0, N, b_is_kn, stream, scatter);
     CUtensorMap a0, b0, b1;
     if ((rc = make_map(&a0, A, K, pb.buffer_rows, 1, BK, BM_CTA)) != MOK_OK) return rc;
     if (!b_is_kn) {
@@ -380,6 +390,7 @@ int launch_gate_up_fused(const GemmProblem& pb, const void* A, int K, const void
     int rc = check_problem(pb);
     if (rc != MOK_OK) return rc;
     if (K <= 0 || N <= 0 || K % BK != 0 || N % BN_CTA != 0 || !Wg || !Wu || !gate || !up || !hidden) return MOK_ERR_INVALID_ARGUMENT;
+    if (pb.occupied_rows != nullptr) return launch_routed_gate_up(pb, A, K, Wg, Wu, gate, up, hidden, N, has_limit, limit, stream);
     CUtensorMap a0, b0, b1;
     if ((rc = make_map(&a0, A, K, pb.buffer_rows, 1, BK, BM_CTA)) != MOK_OK) return rc;
     if ((rc = make_map(&b0, Wg, K, N, pb.num_experts, BK, BN_CTA)) != MOK_OK) return rc;
@@ -398,11 +409,19 @@ int launch_gate_up_fused(const GemmProblem& pb, const void* A, int K, const void
     return launch<MODE_ROWS, false, true>(a0, b0, a0, b1, kp, (window / BM) * kp.n_blocks, stream);
 }
 
+int launch_down_dgrad_fused(const GemmProblem& pb, const void* A, int K, const void* B, const void* gate, const void* up, void* d_hidden,
+                            void* d_gate, void* d_up, float* row_partial, int N, bool has_limit, float limit, cudaStream_t stream) {
+    if (int rc = check_problem(pb)) return rc;
+    if (K <= 0 || N <= 0 || K % BK != 0 || N % BN != 0 || !gate || !up || !d_gate || !d_up || !pb.occupied_rows) return MOK_ERR_INVALID_ARGUMENT;
+    return launch_routed_down_dgrad(pb, A, K, B, gate, up, d_hidden, d_gate, d_up, row_partial, N, has_limit, limit, stream);
+}
+
 int launch_rows_gemm_dual(const GemmProblem& pb, const void* A0, const void* A1, int K, const void* B0, const void* B1,
                           void* D, int N, cudaStream_t stream, const RowScatter* scatter) {
     int rc = check_problem(pb);
     if (rc != MOK_OK) return rc;
     if (K <= 0 || N <= 0 || K % BK != 0 || N % BN != 0) return MOK_ERR_INVALID_ARGUMENT;
+    if (pb.occupied_rows != nullptr) return launch_routed_gemm(pb, A0, A1, K, B0, B1, D, N, true, stream, scatter);
     CUtensorMap a0, a1, b0, b1;
     if ((rc = make_map(&a0, A0, K, pb.buffer_rows, 1, BK, BM_CTA)) != MOK_OK) return rc;
     if ((rc = make_map(&a1, A1, K, pb.buffer_rows, 1, BK, BM_CTA)) != MOK_OK) return rc;

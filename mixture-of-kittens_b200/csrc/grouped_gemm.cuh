@@ -16,8 +16,9 @@ struct GemmProblem {
     int dense_rows = 0;
     int row_begin = 0, row_end = 0;
     int buffer_rows = 0;   // rows of the activation buffers (macrobatch size, or T for a dense problem)
-    // optional, weight-gradient form only: rows of each expert that can be non-zero (the rest of its 256-aligned range
-    // is zero padding); the K loop of expert e ends at this count rounded up to the K step
+    // optional: rows of each expert that can be non-zero (the rest of its 256-aligned range is zero padding).  The K loop of
+    // a weight gradient ends at this count rounded up to the K step; the rows forms of the bf16 GEMM then put the tokens on
+    // the N side of the MMA and leave the padding out (routed_gemm.cu)
     const int32_t* occupied_rows = nullptr;
     uint32_t* status = nullptr;
 };
@@ -44,6 +45,13 @@ int launch_rows_gemm(const GemmProblem& pb, const void* A, int K, const void* B0
 // bf16 [rows, N]) and hidden = silu(gate) * up computed from the stored (rounded) values, optionally clamped.
 int launch_gate_up_fused(const GemmProblem& pb, const void* A, int K, const void* Wg, const void* Wu, void* gate, void* up,
                          void* hidden, int N, bool has_limit, float limit, cudaStream_t stream);
+
+// Input gradient of the down projection with the SwiGLU backward in the epilogue: d_hidden = A * B[e] (B stored [E, K, N])
+// rounded to bf16 and stored (unless nullptr), d_gate / d_up from it and the saved gate / up [rows, N].
+// row_partial (or nullptr): [rows, N / 128] sums of d_hidden * hidden for the router-weight gradient (launch_router_grad).
+// Needs pb.occupied_rows.
+int launch_down_dgrad_fused(const GemmProblem& pb, const void* A, int K, const void* B, const void* gate, const void* up, void* d_hidden,
+                            void* d_gate, void* d_up, float* row_partial, int N, bool has_limit, float limit, cudaStream_t stream);
 
 // D[row, :] = A0[row, :K] * B0[e] + A1[row, :K] * B1[e] with B_s stored [E, K, N] (gate+up input gradient).
 int launch_rows_gemm_dual(const GemmProblem& pb, const void* A0, const void* A1, int K, const void* B0, const void* B1,

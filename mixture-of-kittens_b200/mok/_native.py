@@ -47,7 +47,7 @@ class LayerArgs(ctypes.Structure):
             "hidden_fp8", "hidden_sc", "hidden_fp8_t", "hidden_sc_t", "d_y_fp8", "d_y_sc", "d_y_fp8_t", "d_y_sc_t",
             "d_gate_fp8", "d_gate_sc", "d_up_fp8", "d_up_sc", "d_gate_fp8_t", "d_gate_sc_t", "d_up_fp8_t", "d_up_sc_t",
             "row_source", "unique_peer", "unique_token", "unique_before", "staged_x", "staged_d_y")]
-        + [("staged_rows", c_int), ("reserved1", c_int)]
+        + [("staged_rows", c_int), ("reserved1", c_int), ("occupied_rows", c_void_p), ("row_partials", c_void_p)]
     )
 
 

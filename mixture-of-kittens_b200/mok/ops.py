@@ -470,6 +470,8 @@ def dispatch_mlp_swiglu_combine_fwd_bf16(
     a.x_routed, a.y_routed, a.y_shared = x_routed.data_ptr(), y_routed.data_ptr() or None, y_shared.data_ptr()
     a.gate_shared, a.up_shared, a.hidden_shared = gate_shared.data_ptr(), up_shared.data_ptr(), hidden_shared.data_ptr()
     a.gate_routed, a.up_routed, a.hidden_routed = gate_routed.data_ptr(), up_routed.data_ptr(), hidden_routed.data_ptr()
+    occupied_rows = torch.empty(E, dtype=torch.int32, device=x.device)
+    a.occupied_rows = occupied_rows.data_ptr()
     _staging = _attach_dedup(a, x, cap, ('x',), True, dedup_row_source, dedup_unique_peer, dedup_unique_token,
                              dedup_unique_before)  # noqa: F841  (keeps the staging buffers alive until the launch is queued)
     check(lib().mok_moe_forward_bf16(_native.ctypes.byref(a), stream_ptr(x.device)), "dispatch_mlp_swiglu_combine_fwd_bf16")
@@ -531,6 +533,8 @@ def recompute_forward_context_bf16(
     a.x_routed = x_routed.data_ptr()
     a.gate_shared, a.up_shared, a.hidden_shared = gate_shared.data_ptr(), up_shared.data_ptr(), hidden_shared.data_ptr()
     a.gate_routed, a.up_routed, a.hidden_routed = gate_routed.data_ptr(), up_routed.data_ptr(), hidden_routed.data_ptr()
+    occupied_rows = torch.empty(E, dtype=torch.int32, device=x.device)
+    a.occupied_rows = occupied_rows.data_ptr()
     _staging = _attach_dedup(a, x, cap, ('x',), True, dedup_row_source, dedup_unique_peer, dedup_unique_token,
                              dedup_unique_before)  # noqa: F841  (keeps the staging buffers alive until the launch is queued)
     check(lib().mok_moe_recompute_bf16(_native.ctypes.byref(a), stream_ptr(x.device)), "recompute_forward_context_bf16")
@@ -624,7 +628,7 @@ def dispatch_mlp_swiglu_combine_bwd_bf16(
     d_gate_routed, d_up_routed, d_hidden_routed = new(MB, I), new(MB, I), new(MB, I)
     d_w_shared_gate, d_w_shared_up, d_w_shared_down = new(I, H), new(I, H), new(H, I)
     d_w_routed_gate, d_w_routed_up, d_w_routed_down = new(E, I, H), new(E, I, H), new(E, H, I)
-    row_scratch = torch.empty(2 * MB + E, dtype=torch.float32, device=x.device)
+    row_scratch = torch.empty(2 * MB + E + MB * (I // 128), dtype=torch.float32, device=x.device)
 
     a = _layer_args(ep_size=ep_size, rank=_local_rank(x, x_ptrs), x=x, intermediate=I, num_local_experts=E, topk=topk,
                     capacity=cap, macrobatch_size=MB, minibatch_size=minibatch_size, num_comm_sms=num_comm_sms,
@@ -644,6 +648,7 @@ def dispatch_mlp_swiglu_combine_bwd_bf16(
     a.d_w_shared_gate, a.d_w_shared_up, a.d_w_shared_down = d_w_shared_gate.data_ptr(), d_w_shared_up.data_ptr(), d_w_shared_down.data_ptr()
     a.d_w_routed_gate, a.d_w_routed_up, a.d_w_routed_down = d_w_routed_gate.data_ptr(), d_w_routed_up.data_ptr(), d_w_routed_down.data_ptr()
     a.row_scratch = row_scratch.data_ptr()
+    a.row_partials = row_scratch.data_ptr() + 4 * (2 * MB + E)
     a.d_y_local = d_y_buffer.data_ptr()
     _staging = _attach_dedup(a, x, cap, ('x', 'd_y'), macrobatch_size < cap, dedup_row_source, dedup_unique_peer, dedup_unique_token,
                              dedup_unique_before)  # noqa: F841  (keeps the staging buffers alive until the launch is queued)
