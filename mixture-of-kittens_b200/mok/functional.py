@@ -254,6 +254,20 @@ def _stage(buffer: torch.Tensor, value: torch.Tensor) -> None:
         buffer.copy_(value)
 
 
+def _source(workspace: MoKWorkspace, buffer: torch.Tensor, pointers: list[int], value: torch.Tensor) -> tuple[torch.Tensor, list[int]]:
+    """Where the kernels read an input from, and its address on every rank.  Peers can only reach the symmetric buffer, so
+    with several ranks the input is staged there.  One rank reads the caller's tensor in place, which takes two to seven
+    copies out of every call; inputs that the kernels cannot address (less than 16-byte alignment) or that lie in a buffer
+    the call writes are staged as well, and so is everything while a graph is being traced, where there is no address yet."""
+    if workspace.ep_size == 1 and type(value) in (torch.Tensor, torch.nn.Parameter) and not torch.compiler.is_compiling():
+        address = value.data_ptr()
+        written = (workspace.combine_buffer, workspace.d_x_routed_buffer, workspace.d_router_weight_buffer)
+        if address % 16 == 0 and not any(0 <= address - b.data_ptr() < b.nbytes for b in written):
+            return value, [address]
+    _stage(buffer, value)
+    return buffer, pointers
+
+
 def _scatter_from_gemm(workspace: MoKWorkspace) -> bool:
     """Whether the down projection and the input-gradient GEMM store their rows into the combine slots themselves instead
     of leaving them to a combine pass (the results are the same).  On for one rank, where it saves a read and a write of
@@ -382,8 +396,8 @@ def forward(config: MoKConfig, workspace: MoKWorkspace, schedule: MoKSchedule, x
             swiglu_limit: float | None = None) -> tuple[torch.Tensor, MoKForwardContext]:
     """MoE forward (reference :470-568).  Returns (output bf16 [T, H], forward context for backward)."""
     validate_inputs(config, workspace, schedule, x, router_weights)
-    _stage(workspace.x_buffer, x)
-    _stage(workspace.router_weight_buffer, router_weights)
+    x_in = _source(workspace, workspace.x_buffer, workspace.x_buffer_ptrs, x)
+    weights_in, _ = _source(workspace, workspace.router_weight_buffer, workspace.router_weight_buffer_ptrs, router_weights)
     _barrier(workspace)   # every peer's x is in place before anyone pulls
 
     sched = (schedule.peer_rank, schedule.peer_token_idx, schedule.num_tokens, schedule.tokens_per_expert)
@@ -395,7 +409,7 @@ def forward(config: MoKConfig, workspace: MoKWorkspace, schedule: MoKSchedule, x
         d_fp8, d_sc = routed_down_weights
         (x_t, x_t_sc, gate_shared, gate_q, gate_sc, up_shared, up_q, up_sc, hidden_shared, hid_t, hid_t_sc,
          y_shared, _y_routed) = dispatch_mlp_swiglu_combine_fwd_mxfp8(
-            workspace.x_buffer, workspace.x_buffer_ptrs, workspace.combine_buffer, workspace.combine_buffer_ptrs,
+            *x_in, workspace.combine_buffer, workspace.combine_buffer_ptrs,
             shared_gate_weights, g_fp8, g_sc, shared_up_weights, u_fp8, u_sc, shared_down_weights, d_fp8, d_sc, *sched, *tail)
         context = MoKForwardContext(x_routed=(x_t, x_t_sc), gate_shared=gate_shared, gate_routed=(gate_q, gate_sc),
                                     up_shared=up_shared, up_routed=(up_q, up_sc), hidden_shared=hidden_shared,
@@ -403,14 +417,14 @@ def forward(config: MoKConfig, workspace: MoKWorkspace, schedule: MoKSchedule, x
     else:
         (x_routed, gate_shared, gate_routed, up_shared, up_routed, hidden_shared, hidden_routed, y_shared,
          _y_routed) = dispatch_mlp_swiglu_combine_fwd_bf16(
-            workspace.x_buffer, workspace.x_buffer_ptrs, workspace.combine_buffer, workspace.combine_buffer_ptrs,
+            *x_in, workspace.combine_buffer, workspace.combine_buffer_ptrs,
             shared_gate_weights, routed_gate_weights, shared_up_weights, routed_up_weights,
             shared_down_weights, routed_down_weights, *sched, *tail)
         context = MoKForwardContext(x_routed=x_routed, gate_shared=gate_shared, gate_routed=gate_routed, up_shared=up_shared,
                                     up_routed=up_routed, hidden_shared=hidden_shared, hidden_routed=hidden_routed)
 
     _barrier(workspace)   # every peer's pushes into this rank's combine buffer have landed
-    output = fwd_epilogue(y_shared, workspace.combine_buffer, workspace.router_weight_buffer)
+    output = fwd_epilogue(y_shared, workspace.combine_buffer, weights_in)
     return output, context
 
 
@@ -425,7 +439,7 @@ def recompute_forward_context(config: MoKConfig, workspace: MoKWorkspace, schedu
         raise TypeError("routed gate and up weights must use the same precision representation")
     if isinstance(routed_gate_weights, tuple) and (len(routed_gate_weights) != 2 or len(routed_up_weights) != 2):
         raise ValueError("MXFP8 routed gate and up weights must be data/scale pairs")
-    _stage(workspace.x_buffer, x)
+    x_in = _source(workspace, workspace.x_buffer, workspace.x_buffer_ptrs, x)
     _barrier(workspace)
 
     sched = (schedule.peer_rank, schedule.peer_token_idx, schedule.num_tokens, schedule.tokens_per_expert)
@@ -435,12 +449,12 @@ def recompute_forward_context(config: MoKConfig, workspace: MoKWorkspace, schedu
         g_fp8, g_sc = routed_gate_weights
         u_fp8, u_sc = routed_up_weights
         (x_t, x_t_sc, gate_shared, gate_q, gate_sc, up_shared, up_q, up_sc, hidden_shared, hid_t,
-         hid_t_sc) = recompute_forward_context_mxfp8(workspace.x_buffer, workspace.x_buffer_ptrs, shared_gate_weights, g_fp8, g_sc,
+         hid_t_sc) = recompute_forward_context_mxfp8(*x_in, shared_gate_weights, g_fp8, g_sc,
                                                      shared_up_weights, u_fp8, u_sc, *sched, *tail)
         x_routed, gate_routed, up_routed, hidden_routed = (x_t, x_t_sc), (gate_q, gate_sc), (up_q, up_sc), (hid_t, hid_t_sc)
     else:
         (x_routed, gate_shared, gate_routed, up_shared, up_routed, hidden_shared,
-         hidden_routed) = recompute_forward_context_bf16(workspace.x_buffer, workspace.x_buffer_ptrs, shared_gate_weights,
+         hidden_routed) = recompute_forward_context_bf16(*x_in, shared_gate_weights,
                                                          routed_gate_weights, shared_up_weights, routed_up_weights, *sched, *tail)
     _barrier(workspace)
     return MoKForwardContext(x_routed=x_routed, gate_shared=gate_shared, gate_routed=gate_routed, up_shared=up_shared,
@@ -466,13 +480,12 @@ def backward(config: MoKConfig, workspace: MoKWorkspace, schedule: MoKSchedule, 
     validate_inputs(config, workspace, schedule, x, router_weights, grad_output)
     if not isinstance(forward_context, MoKForwardContext):
         raise TypeError("forward_context must be a MoKForwardContext")
-    _stage(workspace.d_y_buffer, grad_output)
-    _stage(workspace.x_buffer, x)
-    _stage(workspace.router_weight_buffer, router_weights)
+    d_y_in = _source(workspace, workspace.d_y_buffer, workspace.d_y_buffer_ptrs, grad_output)
+    x_in = _source(workspace, workspace.x_buffer, workspace.x_buffer_ptrs, x)
+    weights_in = _source(workspace, workspace.router_weight_buffer, workspace.router_weight_buffer_ptrs, router_weights)
     _barrier(workspace)
 
-    bufs = (workspace.d_y_buffer, workspace.d_y_buffer_ptrs, workspace.d_x_routed_buffer, workspace.d_x_routed_buffer_ptrs,
-            workspace.router_weight_buffer, workspace.router_weight_buffer_ptrs,
+    bufs = (*d_y_in, workspace.d_x_routed_buffer, workspace.d_x_routed_buffer_ptrs, *weights_in,
             workspace.d_router_weight_buffer, workspace.d_router_weight_buffer_ptrs)
     sched = (schedule.peer_rank, schedule.peer_token_idx, schedule.num_tokens, schedule.tokens_per_expert)
     tail = (workspace.topk, swiglu_limit, config.bwd_num_comm_sms, config.macrobatch_size, config.minibatch_size,
@@ -485,7 +498,7 @@ def backward(config: MoKConfig, workspace: MoKWorkspace, schedule: MoKSchedule, 
         out = dispatch_mlp_swiglu_combine_bwd_mxfp8(
             *bufs, shared_gate_weights, g_t_fp8, g_t_sc, shared_up_weights, u_t_fp8, u_t_sc, shared_down_weights, d_t_fp8, d_t_sc,
             *ctx.x_routed, ctx.gate_shared, *ctx.gate_routed, ctx.up_shared, *ctx.up_routed, ctx.hidden_shared, *ctx.hidden_routed,
-            workspace.x_buffer, workspace.x_buffer_ptrs, g_fp8, g_sc, u_fp8, u_sc, *sched, *tail)
+            *x_in, g_fp8, g_sc, u_fp8, u_sc, *sched, *tail)
         d_x_shared = out[0]
         d_w_shared_gate, d_w_routed_gate, d_w_shared_up, d_w_routed_up, d_w_shared_down, d_w_routed_down = out[12:18]
     else:
@@ -493,7 +506,7 @@ def backward(config: MoKConfig, workspace: MoKWorkspace, schedule: MoKSchedule, 
             *bufs, shared_gate_weights, routed_gate_weights, shared_up_weights, routed_up_weights,
             shared_down_weights, routed_down_weights,
             ctx.x_routed, ctx.gate_shared, ctx.gate_routed, ctx.up_shared, ctx.up_routed, ctx.hidden_shared, ctx.hidden_routed,
-            workspace.x_buffer, workspace.x_buffer_ptrs, *sched, *tail)
+            *x_in, *sched, *tail)
         d_x_shared = out[0]
         d_w_shared_gate, d_w_routed_gate, d_w_shared_up, d_w_routed_up, d_w_shared_down, d_w_routed_down = out[9:15]
 
