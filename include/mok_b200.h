@@ -36,7 +36,7 @@ enum {
     MOK_STATUS_BARRIER_TIMEOUT = 2u,     /* a cross-GPU barrier wait ran out */
     MOK_STATUS_PIPELINE_TIMEOUT = 4u,    /* an mbarrier wait inside a GEMM kernel ran out */
     MOK_STATUS_BAD_SCHEDULE_ENTRY = 8u   /* a schedule row named a peer or token outside the buffers (skipped), or the
-                                              schedule claims more rows than the routes padded per expert can fill */
+                                              schedule claims more rows than mok_layer_args.schedule_rows promised */
 };
 
 #define MOK_MAX_EP 8
@@ -267,7 +267,11 @@ typedef struct mok_layer_args {
     const int32_t *row_source, *unique_peer, *unique_token, *unique_before;
     void *staged_x, *staged_d_y;
     int staged_rows;
-    int reserved1;
+    /* Most rows that the schedule claims in num_tokens (a multiple of 256), where the caller knows it: launches then end there
+     * instead of at schedule_capacity, and a schedule that claims more sets MOK_STATUS_BAD_SCHEDULE_ENTRY.  A mok_schedule
+     * result never claims more than (ep_size * T * K + 255 * num_local_experts) / 256 * 256.  0: any number of rows up to
+     * schedule_capacity, however the experts are padded. */
+    int schedule_rows;
     /* Optional scratch of the bf16 calls, used when the experts hold few rows each (NULL: padding rows are computed too). */
     int32_t* occupied_rows;   /* forward, recompute: int32 [num_local_experts] (the backward has room for this in row_scratch) */
     float* row_partials;      /* backward: fp32 [MB * intermediate / 128]; the SwiGLU backward then runs in the epilogue of the

@@ -159,6 +159,7 @@ int check_common(const mok_layer_args* a, bool fp8 = false) {
     if (a->num_local_experts > MOK_MAX_LOCAL_EXPERTS) return MOK_ERR_TOO_LARGE;
     if (a->topk < 1 || a->topk > 255) return MOK_ERR_INVALID_ARGUMENT;
     if (a->schedule_capacity <= 0 || a->schedule_capacity % 256 != 0) return MOK_ERR_INVALID_ARGUMENT;
+    if (a->schedule_rows < 0 || a->schedule_rows % 256 != 0) return MOK_ERR_INVALID_ARGUMENT;
     if (a->minibatch_size <= 0 || a->minibatch_size % 256 != 0) return MOK_ERR_INVALID_ARGUMENT;
     if (a->macrobatch_size <= 0 || a->macrobatch_size % a->minibatch_size != 0) return MOK_ERR_INVALID_ARGUMENT;
     if (a->num_comm_sms <= 0) return MOK_ERR_INVALID_ARGUMENT;
@@ -172,13 +173,12 @@ int check_common(const mok_layer_args* a, bool fp8 = false) {
     return MOK_OK;
 }
 
-// Schedule rows that can carry work: every route once, every local expert padded to 256 rows.  The capacity is at least
-// twice the routes of a rank, so launches sized for it find nothing to do in half of the windows and chunks (each costs
-// the host about 5 us and the GPU 2 to 3).  A schedule that was not built by mok_schedule and claims more rows than this
-// sets MOK_STATUS_BAD_SCHEDULE_ENTRY (dispatch_kernel).
+// Schedule rows that the call runs over.  The capacity is at least twice the routes of a rank, so launches sized for it find
+// nothing to do in half of the windows and chunks (each costs the host about 5 us and the GPU 2 to 3).  How far an expert is
+// padded is the schedule's own business, so only the caller can promise fewer rows; dispatch_kernel and the gathering quantizer
+// report a schedule that claims more.
 int covered_rows(const mok_layer_args* a) {
-    const long long most = (static_cast<long long>(a->ep_size) * a->num_local_tokens * a->topk + 255LL * a->num_local_experts) / 256 * 256;
-    return static_cast<int>(most < a->schedule_capacity ? most : a->schedule_capacity);
+    return a->schedule_rows > 0 && a->schedule_rows < a->schedule_capacity ? a->schedule_rows : a->schedule_capacity;
 }
 
 int num_windows(const mok_layer_args* a) { return (covered_rows(a) + a->macrobatch_size - 1) / a->macrobatch_size; }

@@ -73,7 +73,7 @@ def _(x, x_ptrs, combine_buffer, combine_buffer_ptrs, w_shared_gate, w_routed_ga
       w_routed_up, w_routed_up_sc, w_shared_down, w_routed_down, w_routed_down_sc, schedule_peer_rank,
       schedule_peer_token_idx, num_tokens, tokens_per_expert, topk, swiglu_limit, num_comm_sms, macrobatch_size,
       minibatch_size, dedup_row_source=None, dedup_unique_peer=None,
-      dedup_unique_token=None, dedup_unique_before=None, skip_routed_output=False):
+      dedup_unique_token=None, dedup_unique_before=None, skip_routed_output=False, schedule_rows=0):
     return _fwd_mxfp8_context(x, w_shared_gate, macrobatch_size) + (
         x.new_empty(x.shape), x.new_empty((0 if skip_routed_output else macrobatch_size, x.shape[1])))
 
@@ -82,7 +82,7 @@ def _(x, x_ptrs, combine_buffer, combine_buffer_ptrs, w_shared_gate, w_routed_ga
 def _(x, x_ptrs, combine_buffer, combine_buffer_ptrs, w_shared_gate, w_routed_gate, w_shared_up, w_routed_up,
       w_shared_down, w_routed_down, schedule_peer_rank, schedule_peer_token_idx, num_tokens, tokens_per_expert, topk,
       swiglu_limit, num_comm_sms, macrobatch_size, minibatch_size, dedup_row_source=None, dedup_unique_peer=None,
-      dedup_unique_token=None, dedup_unique_before=None, skip_routed_output=False):
+      dedup_unique_token=None, dedup_unique_before=None, skip_routed_output=False, schedule_rows=0):
     return _fwd_bf16_context(x, w_shared_gate, macrobatch_size) + (
         x.new_empty(x.shape), x.new_empty((0 if skip_routed_output else macrobatch_size, x.shape[1])))
 
@@ -91,14 +91,14 @@ def _(x, x_ptrs, combine_buffer, combine_buffer_ptrs, w_shared_gate, w_routed_ga
 def _(x, x_ptrs, w_shared_gate, w_routed_gate, w_routed_gate_sc, w_shared_up, w_routed_up, w_routed_up_sc,
       schedule_peer_rank, schedule_peer_token_idx, num_tokens, tokens_per_expert, topk, swiglu_limit, num_comm_sms,
       macrobatch_size, minibatch_size, dedup_row_source=None, dedup_unique_peer=None,
-      dedup_unique_token=None, dedup_unique_before=None):
+      dedup_unique_token=None, dedup_unique_before=None, schedule_rows=0):
     return _fwd_mxfp8_context(x, w_shared_gate, macrobatch_size)
 
 
 @torch.library.register_fake("mok::recompute_forward_context_bf16")
 def _(x, x_ptrs, w_shared_gate, w_routed_gate, w_shared_up, w_routed_up, schedule_peer_rank, schedule_peer_token_idx,
       num_tokens, tokens_per_expert, topk, swiglu_limit, num_comm_sms, macrobatch_size, minibatch_size, dedup_row_source=None, dedup_unique_peer=None,
-      dedup_unique_token=None, dedup_unique_before=None):
+      dedup_unique_token=None, dedup_unique_before=None, schedule_rows=0):
     return _fwd_bf16_context(x, w_shared_gate, macrobatch_size)
 
 
@@ -115,7 +115,7 @@ def _(d_y_buffer, d_y_buffer_ptrs, d_x_routed_buffer, d_x_routed_buffer_ptrs, ro
       up_fp8_routed, up_sc_routed, hidden_shared, hidden_fp8_t_routed, hidden_sc_t_routed, x, x_ptrs, w_routed_gate,
       w_routed_gate_sc, w_routed_up, w_routed_up_sc, schedule_peer_rank, schedule_peer_token_idx, num_tokens,
       tokens_per_expert, topk, swiglu_limit, num_comm_sms, macrobatch_size, minibatch_size, dedup_row_source=None, dedup_unique_peer=None,
-      dedup_unique_token=None, dedup_unique_before=None, skip_routed_output=False):
+      dedup_unique_token=None, dedup_unique_before=None, skip_routed_output=False, schedule_rows=0):
     d = d_y_buffer
     t, h = d.shape
     i = w_shared_gate.shape[0]
@@ -133,7 +133,7 @@ def _(d_y_buffer, d_y_buffer_ptrs, d_x_routed_buffer, d_x_routed_buffer_ptrs, ro
       w_shared_up, w_routed_up, w_shared_down, w_routed_down, x_routed, gate_shared, gate_routed, up_shared, up_routed,
       hidden_shared, hidden_routed, x, x_ptrs, schedule_peer_rank, schedule_peer_token_idx, num_tokens,
       tokens_per_expert, topk, swiglu_limit, num_comm_sms, macrobatch_size, minibatch_size, dedup_row_source=None, dedup_unique_peer=None,
-      dedup_unique_token=None, dedup_unique_before=None, skip_routed_output=False):
+      dedup_unique_token=None, dedup_unique_before=None, skip_routed_output=False, schedule_rows=0):
     d = d_y_buffer
     t, h = d.shape
     i = w_shared_gate.shape[0]

@@ -20,7 +20,7 @@ STATUS_BITS = {
     1: "schedule overflow: padded routes exceed schedule_capacity (raise schedule_capacity_multiplier)",
     2: "cross-GPU barrier wait ran out",
     4: "a GEMM pipeline wait ran out",
-    8: "a schedule row named a peer or token outside the buffers, or the schedule claims more rows than its routes fill",
+    8: "a schedule row named a peer or token outside the buffers, or the schedule claims more rows than were promised",
 }
 MAX_EP = 8
 
@@ -47,7 +47,7 @@ class LayerArgs(ctypes.Structure):
             "hidden_fp8", "hidden_sc", "hidden_fp8_t", "hidden_sc_t", "d_y_fp8", "d_y_sc", "d_y_fp8_t", "d_y_sc_t",
             "d_gate_fp8", "d_gate_sc", "d_up_fp8", "d_up_sc", "d_gate_fp8_t", "d_gate_sc_t", "d_up_fp8_t", "d_up_sc_t",
             "row_source", "unique_peer", "unique_token", "unique_before", "staged_x", "staged_d_y")]
-        + [("staged_rows", c_int), ("reserved1", c_int), ("occupied_rows", c_void_p), ("row_partials", c_void_p)]
+        + [("staged_rows", c_int), ("schedule_rows", c_int), ("occupied_rows", c_void_p), ("row_partials", c_void_p)]
     )
 
 

@@ -60,6 +60,9 @@ class MoKSchedule:                     # reference :34-39
     unique_token: torch.Tensor | None = None    # (U,) int32 its token index on that rank
     unique_before: torch.Tensor | None = None   # (schedule_capacity / 256 + 1,) int32 tokens first used below row 256 * i
     num_unique: torch.Tensor | None = None      # (1,) int32
+    # Most rows that the schedule can claim; the layer calls end their launches there.  Set by `build_schedule` alone: a schedule
+    # that a caller puts together, or changes with `dataclasses.replace`, may pad its experts as it likes (0 = no bound known).
+    max_rows: int = field(default=0, init=False)
 
 
 @dataclass(frozen=True, slots=True)
@@ -276,6 +279,10 @@ def _scatter_from_gemm(workspace: MoKWorkspace) -> bool:
     return workspace.ep_size == 1
 
 
+def _schedule_rows(schedule: MoKSchedule) -> int:
+    return getattr(schedule, "max_rows", 0)   # absent in schedules that were pickled before the field existed
+
+
 def _barrier(workspace: MoKWorkspace) -> None:
     if workspace.ep_size == 1:
         return   # nobody to wait for: stream order is enough, and five dispatcher round trips a training step are not free
@@ -354,14 +361,15 @@ def build_schedule(workspace: MoKWorkspace, config: MoKConfig, top_experts: torc
     _barrier(workspace)
     peer_rank, peer_token_idx, num_tokens, tokens_per_expert = schedule(
         workspace.all_gather_top_experts_buffer, num_local_experts, workspace.schedule_capacity, workspace.ep_rank)
-    if not _dedup_wanted(workspace):
-        return MoKSchedule(peer_rank=peer_rank, peer_token_idx=peer_token_idx, num_tokens=num_tokens,
-                           tokens_per_expert=tokens_per_expert)
-    row_source, unique_peer, unique_token, unique_before, num_unique = schedule_dedup(
-        workspace.all_gather_top_experts_buffer, peer_rank, peer_token_idx, num_tokens, num_local_experts, workspace.ep_rank)
-    return MoKSchedule(peer_rank=peer_rank, peer_token_idx=peer_token_idx, num_tokens=num_tokens,
-                       tokens_per_expert=tokens_per_expert, row_source=row_source, unique_peer=unique_peer,
-                       unique_token=unique_token, unique_before=unique_before, num_unique=num_unique)
+    dedup = ()
+    if _dedup_wanted(workspace):
+        dedup = schedule_dedup(workspace.all_gather_top_experts_buffer, peer_rank, peer_token_idx, num_tokens, num_local_experts,
+                               workspace.ep_rank)
+    result = MoKSchedule(peer_rank, peer_token_idx, num_tokens, tokens_per_expert, *dedup)
+    # every route once, every local expert padded to 256 rows
+    routes_max = workspace.ep_size * workspace.num_local_tokens * workspace.topk
+    object.__setattr__(result, "max_rows", (routes_max + 255 * num_local_experts) // 256 * 256)
+    return result
 
 
 def validate_inputs(config: MoKConfig, workspace: MoKWorkspace, schedule: MoKSchedule, x: torch.Tensor,
@@ -402,7 +410,8 @@ def forward(config: MoKConfig, workspace: MoKWorkspace, schedule: MoKSchedule, x
 
     sched = (schedule.peer_rank, schedule.peer_token_idx, schedule.num_tokens, schedule.tokens_per_expert)
     tail = (workspace.topk, swiglu_limit, config.fwd_num_comm_sms, config.macrobatch_size, config.minibatch_size,
-            schedule.row_source, schedule.unique_peer, schedule.unique_token, schedule.unique_before, _scatter_from_gemm(workspace))
+            schedule.row_source, schedule.unique_peer, schedule.unique_token, schedule.unique_before, _scatter_from_gemm(workspace),
+            _schedule_rows(schedule))
     if isinstance(routed_gate_weights, tuple):
         g_fp8, g_sc = routed_gate_weights
         u_fp8, u_sc = routed_up_weights
@@ -444,7 +453,8 @@ def recompute_forward_context(config: MoKConfig, workspace: MoKWorkspace, schedu
 
     sched = (schedule.peer_rank, schedule.peer_token_idx, schedule.num_tokens, schedule.tokens_per_expert)
     tail = (workspace.topk, swiglu_limit, config.fwd_num_comm_sms, config.macrobatch_size, config.minibatch_size,
-            schedule.row_source, schedule.unique_peer, schedule.unique_token, schedule.unique_before)
+            schedule.row_source, schedule.unique_peer, schedule.unique_token, schedule.unique_before,
+            _schedule_rows(schedule))
     if isinstance(routed_gate_weights, tuple):
         g_fp8, g_sc = routed_gate_weights
         u_fp8, u_sc = routed_up_weights
@@ -489,7 +499,8 @@ def backward(config: MoKConfig, workspace: MoKWorkspace, schedule: MoKSchedule, 
             workspace.d_router_weight_buffer, workspace.d_router_weight_buffer_ptrs)
     sched = (schedule.peer_rank, schedule.peer_token_idx, schedule.num_tokens, schedule.tokens_per_expert)
     tail = (workspace.topk, swiglu_limit, config.bwd_num_comm_sms, config.macrobatch_size, config.minibatch_size,
-            schedule.row_source, schedule.unique_peer, schedule.unique_token, schedule.unique_before, _scatter_from_gemm(workspace))
+            schedule.row_source, schedule.unique_peer, schedule.unique_token, schedule.unique_before, _scatter_from_gemm(workspace),
+            _schedule_rows(schedule))
     ctx = forward_context
     if isinstance(routed_gate_weights, tuple):
         g_fp8, g_sc, g_t_fp8, g_t_sc = routed_gate_weights

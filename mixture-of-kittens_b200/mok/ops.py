@@ -102,7 +102,10 @@ def _check_bf16_contiguous(named) -> None:
 
 
 def _layer_args(*, ep_size: int, rank: int, x: torch.Tensor, intermediate: int, num_local_experts: int, topk: int,
-                capacity: int, macrobatch_size: int, minibatch_size: int, num_comm_sms: int, swiglu_limit) -> LayerArgs:
+                capacity: int, macrobatch_size: int, minibatch_size: int, num_comm_sms: int, swiglu_limit,
+                schedule_rows: int) -> LayerArgs:
+    _require(type(schedule_rows) is int and schedule_rows >= 0 and schedule_rows % 256 == 0,
+             "schedule_rows must be a nonnegative multiple of 256")
     a = LayerArgs()
     a.ep_size, a.rank = ep_size, rank
     a.num_local_tokens, a.hidden = x.shape
@@ -110,6 +113,7 @@ def _layer_args(*, ep_size: int, rank: int, x: torch.Tensor, intermediate: int, 
     a.num_local_experts = num_local_experts
     a.topk = topk
     a.schedule_capacity = capacity
+    a.schedule_rows = schedule_rows
     a.macrobatch_size = macrobatch_size
     a.minibatch_size = minibatch_size
     a.num_comm_sms = num_comm_sms
@@ -427,6 +431,7 @@ def dispatch_mlp_swiglu_combine_fwd_bf16(
     dedup_unique_token: torch.Tensor | None = None,
     dedup_unique_before: torch.Tensor | None = None,
     skip_routed_output: bool = False,
+    schedule_rows: int = 0,
 ) -> tuple[torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor,
            torch.Tensor]:
     """BF16 forward: dispatch, routed + shared SwiGLU FFN, combine into the owners' slot buffers.
@@ -434,6 +439,9 @@ def dispatch_mlp_swiglu_combine_fwd_bf16(
     Outputs: x_routed [MB,H], gate_shared [T,I], gate_routed [MB,I], up_shared, up_routed, hidden_shared,
              hidden_routed, y_shared [T,H], y_routed [MB,H]  (all bfloat16)
     With skip_routed_output the down projection stores its rows straight into the combine slots and y_routed is [0,H].
+    schedule_rows: the most rows that num_tokens can hold, where the caller knows (a `schedule` result never has more than
+    (ep_size * T * topk + 255 * E) // 256 * 256); a schedule with more is reported.  0: any number up to the schedule's length,
+    however far its experts are padded.  The other layer ops take it too.
     """
     T, H, I, E = _check_activation_dims(x, w_shared_gate, w_routed_gate)
     _check_layer_scalars(topk, swiglu_limit, num_comm_sms, macrobatch_size, minibatch_size)
@@ -461,7 +469,7 @@ def dispatch_mlp_swiglu_combine_fwd_bf16(
 
     a = _layer_args(ep_size=ep_size, rank=_local_rank(x, x_ptrs), x=x, intermediate=I, num_local_experts=E, topk=topk,
                     capacity=cap, macrobatch_size=macrobatch_size, minibatch_size=minibatch_size,
-                    num_comm_sms=num_comm_sms, swiglu_limit=swiglu_limit)
+                    num_comm_sms=num_comm_sms, swiglu_limit=swiglu_limit, schedule_rows=schedule_rows)
     _keep(a, x_ptrs=x_ptrs, combine_ptrs=combine_buffer_ptrs)
     a.peer_rank, a.peer_token_idx = schedule_peer_rank.data_ptr(), schedule_peer_token_idx.data_ptr()
     a.num_tokens, a.tokens_per_expert = num_tokens.data_ptr(), tokens_per_expert.data_ptr()
@@ -499,6 +507,7 @@ def recompute_forward_context_bf16(
     dedup_unique_peer: torch.Tensor | None = None,
     dedup_unique_token: torch.Tensor | None = None,
     dedup_unique_before: torch.Tensor | None = None,
+    schedule_rows: int = 0,
 ) -> tuple[torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor]:
     """Rebuilds the saved forward context (first macrobatch) without the down projection and combine.
 
@@ -524,7 +533,7 @@ def recompute_forward_context_bf16(
     gate_routed, up_routed, hidden_routed = new(macrobatch_size, I), new(macrobatch_size, I), new(macrobatch_size, I)
     a = _layer_args(ep_size=ep_size, rank=_local_rank(x, x_ptrs), x=x, intermediate=I, num_local_experts=E, topk=topk,
                     capacity=cap, macrobatch_size=macrobatch_size, minibatch_size=minibatch_size,
-                    num_comm_sms=num_comm_sms, swiglu_limit=swiglu_limit)
+                    num_comm_sms=num_comm_sms, swiglu_limit=swiglu_limit, schedule_rows=schedule_rows)
     _keep(a, x_ptrs=x_ptrs)
     a.peer_rank, a.peer_token_idx = schedule_peer_rank.data_ptr(), schedule_peer_token_idx.data_ptr()
     a.num_tokens, a.tokens_per_expert = num_tokens.data_ptr(), tokens_per_expert.data_ptr()
@@ -583,6 +592,7 @@ def dispatch_mlp_swiglu_combine_bwd_bf16(
     dedup_unique_token: torch.Tensor | None = None,
     dedup_unique_before: torch.Tensor | None = None,
     skip_routed_output: bool = False,
+    schedule_rows: int = 0,
 ) -> tuple[torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor,
            torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor]:
     """BF16 backward of the layer.
@@ -632,7 +642,7 @@ def dispatch_mlp_swiglu_combine_bwd_bf16(
 
     a = _layer_args(ep_size=ep_size, rank=_local_rank(x, x_ptrs), x=x, intermediate=I, num_local_experts=E, topk=topk,
                     capacity=cap, macrobatch_size=MB, minibatch_size=minibatch_size, num_comm_sms=num_comm_sms,
-                    swiglu_limit=swiglu_limit)
+                    swiglu_limit=swiglu_limit, schedule_rows=schedule_rows)
     _keep(a, x_ptrs=x_ptrs, d_y_ptrs=d_y_buffer_ptrs, d_x_routed_ptrs=d_x_routed_buffer_ptrs,
           router_weight_ptrs=router_weight_buffer_ptrs, d_router_weight_ptrs=d_router_weight_buffer_ptrs)
     a.peer_rank, a.peer_token_idx = schedule_peer_rank.data_ptr(), schedule_peer_token_idx.data_ptr()
@@ -736,6 +746,7 @@ def dispatch_mlp_swiglu_combine_fwd_mxfp8(
     dedup_unique_token: torch.Tensor | None = None,
     dedup_unique_before: torch.Tensor | None = None,
     skip_routed_output: bool = False,
+    schedule_rows: int = 0,
 ) -> tuple[torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor,
            torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor]:
     """MXFP8 forward (routed experts in e4m3 with e8m0 block scales, shared expert in bf16).
@@ -775,7 +786,7 @@ def dispatch_mlp_swiglu_combine_fwd_mxfp8(
 
     a = _layer_args(ep_size=ep_size, rank=_local_rank(x, x_ptrs), x=x, intermediate=I, num_local_experts=E, topk=topk,
                     capacity=cap, macrobatch_size=MB, minibatch_size=minibatch_size, num_comm_sms=num_comm_sms,
-                    swiglu_limit=swiglu_limit)
+                    swiglu_limit=swiglu_limit, schedule_rows=schedule_rows)
     _keep(a, x_ptrs=x_ptrs, combine_ptrs=combine_buffer_ptrs)
     _set_ptrs(a, peer_rank=schedule_peer_rank, peer_token_idx=schedule_peer_token_idx, num_tokens=num_tokens,
               tokens_per_expert=tokens_per_expert, w_shared_gate=w_shared_gate, w_shared_up=w_shared_up,
@@ -813,6 +824,7 @@ def recompute_forward_context_mxfp8(
     dedup_unique_peer: torch.Tensor | None = None,
     dedup_unique_token: torch.Tensor | None = None,
     dedup_unique_before: torch.Tensor | None = None,
+    schedule_rows: int = 0,
 ) -> tuple[torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor,
            torch.Tensor, torch.Tensor, torch.Tensor]:
     """MXFP8 context recomputation (first macrobatch): dispatch, quantize, gate / up GEMMs, SwiGLU, quantize.
@@ -845,7 +857,7 @@ def recompute_forward_context_mxfp8(
     hid_q, hid_sc = _new_fp8(x, MB, I)
     a = _layer_args(ep_size=ep_size, rank=_local_rank(x, x_ptrs), x=x, intermediate=I, num_local_experts=E, topk=topk,
                     capacity=cap, macrobatch_size=MB, minibatch_size=minibatch_size, num_comm_sms=num_comm_sms,
-                    swiglu_limit=swiglu_limit)
+                    swiglu_limit=swiglu_limit, schedule_rows=schedule_rows)
     _keep(a, x_ptrs=x_ptrs)
     _set_ptrs(a, peer_rank=schedule_peer_rank, peer_token_idx=schedule_peer_token_idx, num_tokens=num_tokens,
               tokens_per_expert=tokens_per_expert, w_shared_gate=w_shared_gate, w_shared_up=w_shared_up,
@@ -913,6 +925,7 @@ def dispatch_mlp_swiglu_combine_bwd_mxfp8(
     dedup_unique_token: torch.Tensor | None = None,
     dedup_unique_before: torch.Tensor | None = None,
     skip_routed_output: bool = False,
+    schedule_rows: int = 0,
 ) -> tuple[torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor,
            torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor,
            torch.Tensor, torch.Tensor]:
@@ -973,7 +986,7 @@ def dispatch_mlp_swiglu_combine_bwd_mxfp8(
 
     a = _layer_args(ep_size=ep_size, rank=_local_rank(x, x_ptrs), x=x, intermediate=I, num_local_experts=E, topk=topk,
                     capacity=cap, macrobatch_size=MB, minibatch_size=minibatch_size, num_comm_sms=num_comm_sms,
-                    swiglu_limit=swiglu_limit)
+                    swiglu_limit=swiglu_limit, schedule_rows=schedule_rows)
     _keep(a, x_ptrs=x_ptrs, d_y_ptrs=d_y_buffer_ptrs, d_x_routed_ptrs=d_x_routed_buffer_ptrs,
           router_weight_ptrs=router_weight_buffer_ptrs, d_router_weight_ptrs=d_router_weight_buffer_ptrs)
     _set_ptrs(a, peer_rank=schedule_peer_rank, peer_token_idx=schedule_peer_token_idx, num_tokens=num_tokens,
