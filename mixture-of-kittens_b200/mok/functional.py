@@ -257,12 +257,20 @@ def _stage(buffer: torch.Tensor, value: torch.Tensor) -> None:
         buffer.copy_(value)
 
 
+def _traced() -> bool:
+    """Whether the call may be recorded for tensors that do not exist yet (torch.compile, export, make_fx in every mode,
+    torch.jit.trace) or sees wrapped ones (functorch transforms): an address taken now would be no input of the recording."""
+    return (torch.compiler.is_compiling() or torch.jit.is_tracing() or torch._C._len_torch_dispatch_stack() > 0
+            or torch._ops._len_torch_dispatch_stack_pre_dispatch() > 0 or torch._C._functorch.peek_interpreter_stack() is not None)
+
+
 def _source(workspace: MoKWorkspace, buffer: torch.Tensor, pointers: list[int], value: torch.Tensor) -> tuple[torch.Tensor, list[int]]:
     """Where the kernels read an input from, and its address on every rank.  Peers can only reach the symmetric buffer, so
     with several ranks the input is staged there.  One rank reads the caller's tensor in place, which takes two to seven
     copies out of every call; inputs that the kernels cannot address (less than 16-byte alignment) or that lie in a buffer
-    the call writes are staged as well, and so is everything while a graph is being traced, where there is no address yet."""
-    if workspace.ep_size == 1 and type(value) in (torch.Tensor, torch.nn.Parameter) and not torch.compiler.is_compiling():
+    the call writes are staged as well, and so is everything while a graph is being traced, where the address would be
+    recorded as a constant."""
+    if workspace.ep_size == 1 and type(value) in (torch.Tensor, torch.nn.Parameter) and not _traced():
         address = value.data_ptr()
         written = (workspace.combine_buffer, workspace.d_x_routed_buffer, workspace.d_router_weight_buffer)
         if address % 16 == 0 and not any(0 <= address - b.data_ptr() < b.nbytes for b in written):
