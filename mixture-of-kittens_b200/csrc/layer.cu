@@ -22,6 +22,7 @@
 #include "comm.cuh"
 #include "elementwise.cuh"
 #include "grouped_gemm.cuh"
+#include "layer_windows.cuh"
 #include "mxfp8.cuh"
 #include "mxfp8_gemm.cuh"
 
@@ -29,7 +30,6 @@ namespace mok {
 namespace {
 
 constexpr int kMaxEvents = 512;
-constexpr int kMinibatchesPerChunk = 8;
 
 struct DeviceStreams {
     cudaStream_t comm = nullptr;
@@ -128,27 +128,6 @@ bool overlap_enabled() {
     return !(v != nullptr && v[0] == '1');
 }
 
-// Rows handed from dispatch to the GEMMs to combine in one piece: kMinibatchesPerChunk minibatches, so the caller's
-// minibatch_size sets the hand-over granularity (the default 4096 gives 32768-row chunks, the size that measured best
-// on the DeepSeek-V3-shaped layer).  MOK_CHUNK_ROWS overrides the row count (rounded up to whole minibatches).
-// A window is cut into equal chunks of about that size; one that holds less than one and a half of them stays whole.
-// Without anything to hand over (`whole`) it stays whole too: every further launch adds a nearly empty last wave of tiles.
-int chunk_rows_for(const mok_layer_args* a, int window_rows, bool whole) {
-    long long rows = whole ? window_rows : static_cast<long long>(kMinibatchesPerChunk) * a->minibatch_size;
-    if (const char* v = getenv("MOK_CHUNK_ROWS")) {
-        const int r = atoi(v);
-        if (r > 0) rows = r;
-    }
-    const long long n = (window_rows + rows / 2) / rows;
-    if (n <= 1) return window_rows;
-    rows = (window_rows + n - 1) / n;
-    rows = (rows + a->minibatch_size - 1) / a->minibatch_size * a->minibatch_size;
-    // never more than ~100 chunks per window: events and launches stay bounded
-    const long long min_rows = (a->macrobatch_size / 100 + a->minibatch_size) / a->minibatch_size * a->minibatch_size;
-    if (rows < min_rows) rows = min_rows;
-    return static_cast<int>(rows < window_rows ? rows : window_rows);
-}
-
 int check_common(const mok_layer_args* a, bool fp8 = false) {
     if (a == nullptr) return MOK_ERR_INVALID_ARGUMENT;
     if (a->ep_size < 1 || a->ep_size > MOK_MAX_EP || a->rank < 0 || a->rank >= a->ep_size) return MOK_ERR_INVALID_ARGUMENT;
@@ -171,29 +150,6 @@ int check_common(const mok_layer_args* a, bool fp8 = false) {
     if (any_shared && !(a->w_shared_gate && a->w_shared_up && a->gate_shared && a->up_shared && a->hidden_shared))
         return MOK_ERR_INVALID_ARGUMENT;
     return MOK_OK;
-}
-
-// Schedule rows that the call runs over.  The capacity is at least twice the routes of a rank, so launches sized for it find
-// nothing to do in half of the windows and chunks (each costs the host about 5 us and the GPU 2 to 3).  How far an expert is
-// padded is the schedule's own business, so only the caller can promise fewer rows; dispatch_kernel and the gathering quantizer
-// report a schedule that claims more.
-int covered_rows(const mok_layer_args* a) {
-    return a->schedule_rows > 0 && a->schedule_rows < a->schedule_capacity ? a->schedule_rows : a->schedule_capacity;
-}
-
-int num_windows(const mok_layer_args* a) { return (covered_rows(a) + a->macrobatch_size - 1) / a->macrobatch_size; }
-
-// rows [begin, end) of the schedule; `base` is the schedule row held by row 0 of the activation buffers
-struct Span {
-    int begin, end, base;
-};
-
-Span window_span(const mok_layer_args* a, int w) {
-    Span s;
-    s.begin = s.base = w * a->macrobatch_size;
-    s.end = s.begin + a->macrobatch_size;
-    if (s.end > covered_rows(a)) s.end = covered_rows(a);
-    return s;
 }
 
 RowWindow rows_of(const mok_layer_args* a, const Span& s) {
