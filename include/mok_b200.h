@@ -248,7 +248,7 @@ typedef struct mok_layer_args {
     uint32_t* status;      /* uint32 [1] */
     /* MXFP8 entry points only (NULL otherwise).  "fp8" = e4m3 bytes, "sc" = e8m0 scale tiles [rows/128, cols/128, 32, 16]
      * of the matrix as stored (scales along its last dimension).  In the MXFP8 calls the bf16 routed activation
-     * fields above (x_routed ... d_x_routed) are scratch of the same shapes. */
+     * fields above (x_routed ... d_x_routed) are scratch of the same shapes; mok_layer_scratch says which are used. */
     const void *w_gate_fp8, *w_gate_sc, *w_up_fp8, *w_up_sc, *w_down_fp8, *w_down_sc;   /* [E,I,H] [E,I,H] [E,H,I] */
     const void *w_gate_t_fp8, *w_gate_t_sc, *w_up_t_fp8, *w_up_t_sc;                     /* transposes [E,H,I] (backward) */
     const void *w_down_t_fp8, *w_down_t_sc;                                              /* transpose [E,I,H] (backward) */
@@ -277,6 +277,16 @@ typedef struct mok_layer_args {
     float* row_partials;      /* backward: fp32 [MB * intermediate / 128]; the SwiGLU backward then runs in the epilogue of the
                                  down projection's input gradient */
 } mok_layer_args;
+
+/* Scratch that a layer call may or may not use.  mok_layer_scratch answers for the sizes in `args` (no pointer is looked at) and
+ * the switches in the environment; a buffer whose bit is not set may be NULL.  Bits: */
+enum {
+    MOK_SCRATCH_DISPATCHED = 1u,    /* x_routed, and d_y_routed of the backward (outputs of the bf16 calls) */
+    MOK_SCRATCH_ACTIVATIONS = 2u,   /* gate_routed, up_routed, hidden_routed (outputs of the bf16 calls) */
+    MOK_SCRATCH_GRADIENTS = 4u,     /* d_gate_routed, d_up_routed (outputs of the bf16 backward) */
+    MOK_SCRATCH_ROW_PARTIALS = 8u   /* row_partials of the bf16 backward */
+};
+unsigned mok_layer_scratch(const mok_layer_args* args, int mxfp8);
 
 /*
  * BF16 forward: dispatch -> gate/up GEMM -> SwiGLU -> down GEMM -> combine, macrobatches last to first,

@@ -128,6 +128,21 @@ bool overlap_enabled() {
     return !(v != nullptr && v[0] == '1');
 }
 
+bool fused_activations_enabled();
+bool fused_epilogue_enabled();
+bool row_trim_enabled(const mok_layer_args* a);
+bool gathers_in_quantizer(const mok_layer_args* a);
+
+// see mok_layer_scratch
+unsigned scratch_used(const mok_layer_args* a, bool fp8) {
+    if (!fp8) return MOK_SCRATCH_DISPATCHED | MOK_SCRATCH_ACTIVATIONS | MOK_SCRATCH_GRADIENTS | (row_trim_enabled(a) ? MOK_SCRATCH_ROW_PARTIALS : 0u);
+    unsigned used = 0;
+    if (!gathers_in_quantizer(a)) used |= MOK_SCRATCH_DISPATCHED;
+    if (!fused_activations_enabled() || !fused_epilogue_enabled()) used |= MOK_SCRATCH_ACTIVATIONS;
+    if (!fused_activations_enabled()) used |= MOK_SCRATCH_GRADIENTS;
+    return used;
+}
+
 int check_common(const mok_layer_args* a, bool fp8 = false) {
     if (a == nullptr) return MOK_ERR_INVALID_ARGUMENT;
     if (a->ep_size < 1 || a->ep_size > MOK_MAX_EP || a->rank < 0 || a->rank >= a->ep_size) return MOK_ERR_INVALID_ARGUMENT;
@@ -145,7 +160,9 @@ int check_common(const mok_layer_args* a, bool fp8 = false) {
     if (!a->peer_rank || !a->peer_token_idx || !a->num_tokens || !a->tokens_per_expert) return MOK_ERR_INVALID_ARGUMENT;
     if (!a->x_ptrs || !a->x_local) return MOK_ERR_INVALID_ARGUMENT;
     if (!fp8 && (!a->w_routed_gate || !a->w_routed_up)) return MOK_ERR_INVALID_ARGUMENT;
-    if (!a->x_routed || !a->gate_routed || !a->up_routed || !a->hidden_routed) return MOK_ERR_INVALID_ARGUMENT;
+    const unsigned used = scratch_used(a, fp8);
+    if ((used & MOK_SCRATCH_DISPATCHED) && !a->x_routed) return MOK_ERR_INVALID_ARGUMENT;
+    if ((used & MOK_SCRATCH_ACTIVATIONS) && (!a->gate_routed || !a->up_routed || !a->hidden_routed)) return MOK_ERR_INVALID_ARGUMENT;
     const bool any_shared = a->w_shared_gate || a->w_shared_up;
     if (any_shared && !(a->w_shared_gate && a->w_shared_up && a->gate_shared && a->up_shared && a->hidden_shared))
         return MOK_ERR_INVALID_ARGUMENT;
@@ -564,6 +581,8 @@ int run_chunks(const mok_layer_args* a, const Span& win, bool overlapped, Device
 }  // namespace
 }  // namespace mok
 
+extern "C" unsigned mok_layer_scratch(const mok_layer_args* a, int mxfp8) { return a == nullptr ? 0u : mok::scratch_used(a, mxfp8 != 0); }
+
 extern "C" int mok_moe_forward_bf16(const mok_layer_args* a, mok_stream_t stream) {
     using namespace mok;
     MOK_TRY(check_common(a));
@@ -783,9 +802,11 @@ extern "C" int mok_moe_backward_mxfp8(const mok_layer_args* a, mok_stream_t stre
     if (!a->d_y_ptrs || !a->d_x_routed_ptrs || !a->router_weight_ptrs || !a->d_router_weight_ptrs) return MOK_ERR_INVALID_ARGUMENT;
     if (!a->w_gate_t_fp8 || !a->w_gate_t_sc || !a->w_up_t_fp8 || !a->w_up_t_sc || !a->w_down_t_fp8 || !a->w_down_t_sc)
         return MOK_ERR_INVALID_ARGUMENT;
-    if (!a->d_gate_routed || !a->d_up_routed || !a->d_hidden_routed || !a->d_y_routed || !a->d_w_routed_gate ||
-        !a->d_w_routed_up || !a->d_w_routed_down || !a->row_scratch)
+    if (!a->d_hidden_routed || !a->d_w_routed_gate || !a->d_w_routed_up || !a->d_w_routed_down || !a->row_scratch)
         return MOK_ERR_INVALID_ARGUMENT;
+    const unsigned used = scratch_used(a, true);
+    if ((used & MOK_SCRATCH_DISPATCHED) && !a->d_y_routed) return MOK_ERR_INVALID_ARGUMENT;
+    if ((used & MOK_SCRATCH_GRADIENTS) && (!a->d_gate_routed || !a->d_up_routed)) return MOK_ERR_INVALID_ARGUMENT;
     if (!a->d_y_fp8 || !a->d_y_sc || !a->d_y_fp8_t || !a->d_y_sc_t || !a->d_gate_fp8 || !a->d_gate_sc || !a->d_up_fp8 ||
         !a->d_up_sc || !a->d_gate_fp8_t || !a->d_gate_sc_t || !a->d_up_fp8_t || !a->d_up_sc_t)
         return MOK_ERR_INVALID_ARGUMENT;

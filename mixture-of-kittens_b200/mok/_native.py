@@ -23,6 +23,8 @@ STATUS_BITS = {
     8: "a schedule row named a peer or token outside the buffers, or the schedule claims more rows than were promised",
 }
 MAX_EP = 8
+# MOK_SCRATCH_* bits of mok_layer_scratch
+SCRATCH_DISPATCHED, SCRATCH_ACTIVATIONS, SCRATCH_GRADIENTS, SCRATCH_ROW_PARTIALS = 1, 2, 4, 8
 
 
 class LayerArgs(ctypes.Structure):
@@ -63,6 +65,8 @@ def lib() -> ctypes.CDLL:
         L.mok_launch_count.restype = ctypes.c_longlong
         L.mok_schedule_scratch_bytes.restype = c_int64
         L.mok_schedule_scratch_bytes.argtypes = [c_int, c_int, c_int, c_int]
+        L.mok_layer_scratch.argtypes = [POINTER(LayerArgs), c_int]
+        L.mok_layer_scratch.restype = ctypes.c_uint
         L.mok_schedule.argtypes = [c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p,
                                    c_void_p, c_void_p, c_void_p]
         L.mok_schedule_static.argtypes = [c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p,

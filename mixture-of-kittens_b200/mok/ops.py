@@ -148,6 +148,19 @@ def _set_ptrs(args: LayerArgs, **tensors) -> None:
         setattr(args, field, None if tensor is None else tensor.data_ptr() or None)
 
 
+def _bf16_scratch(args: LayerArgs, new, rows: int, backward: bool = False) -> dict[str, torch.Tensor]:
+    """The bf16 scratch [rows, H] / [rows, I] that an MXFP8 call uses (none of it with one rank and the fused kernels)."""
+    used, H, I = lib().mok_layer_scratch(_native.ctypes.byref(args), 1), args.hidden, args.intermediate
+    scratch = {}
+    if used & _native.SCRATCH_DISPATCHED:
+        scratch.update({n: new(rows, H) for n in (("x_routed", "d_y_routed") if backward else ("x_routed",))})
+    if used & _native.SCRATCH_ACTIVATIONS:
+        scratch.update({n: new(rows, I) for n in ("gate_routed", "up_routed", "hidden_routed")})
+    if backward and used & _native.SCRATCH_GRADIENTS:
+        scratch.update({n: new(rows, I) for n in ("d_gate_routed", "d_up_routed")})
+    return scratch
+
+
 def _new_fp8(like: torch.Tensor, rows: int, cols: int):
     """An e4m3 [rows, cols] buffer and its e8m0 scale tiles [rows/128, cols/128, 32, 16]."""
     return (like.new_empty((rows, cols), dtype=torch.float8_e4m3fn),
@@ -638,11 +651,12 @@ def dispatch_mlp_swiglu_combine_bwd_bf16(
     d_gate_routed, d_up_routed, d_hidden_routed = new(MB, I), new(MB, I), new(MB, I)
     d_w_shared_gate, d_w_shared_up, d_w_shared_down = new(I, H), new(I, H), new(H, I)
     d_w_routed_gate, d_w_routed_up, d_w_routed_down = new(E, I, H), new(E, I, H), new(E, H, I)
-    row_scratch = torch.empty(2 * MB + E + MB * (I // 128), dtype=torch.float32, device=x.device)
 
     a = _layer_args(ep_size=ep_size, rank=_local_rank(x, x_ptrs), x=x, intermediate=I, num_local_experts=E, topk=topk,
                     capacity=cap, macrobatch_size=MB, minibatch_size=minibatch_size, num_comm_sms=num_comm_sms,
                     swiglu_limit=swiglu_limit, schedule_rows=schedule_rows)
+    partials = lib().mok_layer_scratch(_native.ctypes.byref(a), 0) & _native.SCRATCH_ROW_PARTIALS
+    row_scratch = torch.empty(2 * MB + E + (MB * (I // 128) if partials else 0), dtype=torch.float32, device=x.device)
     _keep(a, x_ptrs=x_ptrs, d_y_ptrs=d_y_buffer_ptrs, d_x_routed_ptrs=d_x_routed_buffer_ptrs,
           router_weight_ptrs=router_weight_buffer_ptrs, d_router_weight_ptrs=d_router_weight_buffer_ptrs)
     a.peer_rank, a.peer_token_idx = schedule_peer_rank.data_ptr(), schedule_peer_token_idx.data_ptr()
@@ -658,7 +672,7 @@ def dispatch_mlp_swiglu_combine_bwd_bf16(
     a.d_w_shared_gate, a.d_w_shared_up, a.d_w_shared_down = d_w_shared_gate.data_ptr(), d_w_shared_up.data_ptr(), d_w_shared_down.data_ptr()
     a.d_w_routed_gate, a.d_w_routed_up, a.d_w_routed_down = d_w_routed_gate.data_ptr(), d_w_routed_up.data_ptr(), d_w_routed_down.data_ptr()
     a.row_scratch = row_scratch.data_ptr()
-    a.row_partials = row_scratch.data_ptr() + 4 * (2 * MB + E)
+    a.row_partials = row_scratch.data_ptr() + 4 * (2 * MB + E) if partials else None
     a.d_y_local = d_y_buffer.data_ptr()
     _staging = _attach_dedup(a, x, cap, ('x', 'd_y'), macrobatch_size < cap, dedup_row_source, dedup_unique_peer, dedup_unique_token,
                              dedup_unique_before)  # noqa: F841  (keeps the staging buffers alive until the launch is queued)
@@ -780,13 +794,13 @@ def dispatch_mlp_swiglu_combine_fwd_mxfp8(
     hid_t, hid_t_sc = _new_fp8(x, I, MB)
     gate_shared, up_shared, hidden_shared, y_shared = new(T, I), new(T, I), new(T, I), new(T, H)
     y_routed = new(0 if skip_routed_output else MB, H)
-    scratch = dict(x_routed=new(MB, H), gate_routed=new(MB, I), up_routed=new(MB, I), hidden_routed=new(MB, I))
     x_q, x_sc = _new_fp8(x, MB, H)
     hid_q, hid_sc = _new_fp8(x, MB, I)
 
     a = _layer_args(ep_size=ep_size, rank=_local_rank(x, x_ptrs), x=x, intermediate=I, num_local_experts=E, topk=topk,
                     capacity=cap, macrobatch_size=MB, minibatch_size=minibatch_size, num_comm_sms=num_comm_sms,
                     swiglu_limit=swiglu_limit, schedule_rows=schedule_rows)
+    scratch = _bf16_scratch(a, new, MB)
     _keep(a, x_ptrs=x_ptrs, combine_ptrs=combine_buffer_ptrs)
     _set_ptrs(a, peer_rank=schedule_peer_rank, peer_token_idx=schedule_peer_token_idx, num_tokens=num_tokens,
               tokens_per_expert=tokens_per_expert, w_shared_gate=w_shared_gate, w_shared_up=w_shared_up,
@@ -852,12 +866,12 @@ def recompute_forward_context_mxfp8(
     up_q, up_sc = _new_fp8(x, MB, I)
     hid_t, hid_t_sc = _new_fp8(x, I, MB)
     gate_shared, up_shared, hidden_shared = new(T, I), new(T, I), new(T, I)
-    scratch = dict(x_routed=new(MB, H), gate_routed=new(MB, I), up_routed=new(MB, I), hidden_routed=new(MB, I))
     x_q, x_sc = _new_fp8(x, MB, H)
     hid_q, hid_sc = _new_fp8(x, MB, I)
     a = _layer_args(ep_size=ep_size, rank=_local_rank(x, x_ptrs), x=x, intermediate=I, num_local_experts=E, topk=topk,
                     capacity=cap, macrobatch_size=MB, minibatch_size=minibatch_size, num_comm_sms=num_comm_sms,
                     swiglu_limit=swiglu_limit, schedule_rows=schedule_rows)
+    scratch = _bf16_scratch(a, new, MB)
     _keep(a, x_ptrs=x_ptrs)
     _set_ptrs(a, peer_rank=schedule_peer_rank, peer_token_idx=schedule_peer_token_idx, num_tokens=num_tokens,
               tokens_per_expert=tokens_per_expert, w_shared_gate=w_shared_gate, w_shared_up=w_shared_up,
@@ -975,8 +989,6 @@ def dispatch_mlp_swiglu_combine_bwd_mxfp8(
     d_y_q, d_y_sc = _new_fp8(x, MB, H)
     d_w_shared_gate, d_w_shared_up, d_w_shared_down = new(I, H), new(I, H), new(H, I)
     d_w_routed_gate, d_w_routed_up, d_w_routed_down = new(E, I, H), new(E, I, H), new(E, H, I)
-    scratch = dict(x_routed=new(MB, H), gate_routed=new(MB, I), up_routed=new(MB, I), hidden_routed=new(MB, I),
-                   d_y_routed=new(MB, H), d_gate_routed=new(MB, I), d_up_routed=new(MB, I))
     x_q, x_sc = _new_fp8(x, MB, H)
     hid_q, hid_sc = _new_fp8(x, MB, I)
     d_y_t, d_y_t_sc = _new_fp8(x, H, MB)
@@ -987,6 +999,7 @@ def dispatch_mlp_swiglu_combine_bwd_mxfp8(
     a = _layer_args(ep_size=ep_size, rank=_local_rank(x, x_ptrs), x=x, intermediate=I, num_local_experts=E, topk=topk,
                     capacity=cap, macrobatch_size=MB, minibatch_size=minibatch_size, num_comm_sms=num_comm_sms,
                     swiglu_limit=swiglu_limit, schedule_rows=schedule_rows)
+    scratch = _bf16_scratch(a, new, MB, backward=True)
     _keep(a, x_ptrs=x_ptrs, d_y_ptrs=d_y_buffer_ptrs, d_x_routed_ptrs=d_x_routed_buffer_ptrs,
           router_weight_ptrs=router_weight_buffer_ptrs, d_router_weight_ptrs=d_router_weight_buffer_ptrs)
     _set_ptrs(a, peer_rank=schedule_peer_rank, peer_token_idx=schedule_peer_token_idx, num_tokens=num_tokens,
