@@ -3,6 +3,8 @@
 // CTA-pair launch, argument checks).
 #pragma once
 
+#include <cstdlib>
+
 #include "grouped_gemm.cuh"
 
 namespace mok {
@@ -291,7 +293,14 @@ inline KernelParams base_params(const GemmProblem& pb) {
 // backward of 16384 tokens: 50.5 ms m tile major, 47.5 / 47.0 / 46.8 ms in groups of 4 / 8 / 16.  At 59 MB and below
 // (hidden 7168, intermediate 2048) all widths were within 1 % (m tile major ahead by 0.7 % in MXFP8), so the line is
 // drawn between the two, at half of the 126 MB L2: a line read by SMs of both dies takes room on each.
-inline int rows_group(long long expert_weight_bytes) { return expert_weight_bytes > (63LL << 20) ? kRowsGroup : 1; }
+// MOK_ROWS_GROUP=n sets the width, for measurements and tests (same results).
+inline int rows_group(long long expert_weight_bytes) {
+    if (const char* v = std::getenv("MOK_ROWS_GROUP")) {
+        const int width = std::atoi(v);
+        if (width > 0 && width <= 1024) return width;
+    }
+    return expert_weight_bytes > (63LL << 20) ? kRowsGroup : 1;
+}
 
 // Launches `kernel` as clusters of two CTAs, as many pairs as can be resident at once (at most one per tile).
 // `resident_pairs` caches the occupancy query per device and kernel instantiation.
