@@ -43,8 +43,8 @@ def test_schedule_that_claims_more_rows_is_reported(dist_ctx):
 
 
 @pytest.mark.parametrize("mxfp8", [False, True])
-@pytest.mark.parametrize("T,K,E", [(1024, 2, 3), (512, 1, 8)])   # GEMMs over the padding rows, and without them
-def test_experts_padded_to_a_fixed_capacity(dist_ctx, monkeypatch, T, K, E, mxfp8):
+@pytest.mark.parametrize("T,K,E,no_trim", [(1024, 2, 3, "1"), (512, 1, 8, "0")])   # GEMMs over the padding rows, and without them
+def test_experts_padded_to_a_fixed_capacity(dist_ctx, monkeypatch, T, K, E, no_trim, mxfp8):
     """A schedule that did not come from `schedule` may pad its experts as it likes: with 1024 rows per expert, nearly all of
     them padding, slots, outputs and gradients are bitwise those of the compact schedule, through the functional calls and
     the ops, in several windows (an expert each, so that no gradient is a sum over windows)."""
@@ -53,6 +53,7 @@ def test_experts_padded_to_a_fixed_capacity(dist_ctx, monkeypatch, T, K, E, mxfp
     import torch.distributed as dist
     import mok
     F, dev, cap_e = mok.functional, dist_ctx[2], 1024
+    monkeypatch.setenv("MOK_NO_ROW_TRIM", no_trim)
     inp = O.make_rank_inputs(0, E, E, K, T, 256, 256)
     d = {k: v.to(dev) for k, v in vars(inp).items()}
     routed = [d[n] for n in ("w_routed_gate", "w_routed_up", "w_routed_down")]

@@ -4,10 +4,10 @@ import pytest
 import torch
 
 
-def _args(T, K, E, ep=1):
+def _args(T, K, E, ep=1, H=2048, I=2048):
     from mok import _native as nat
     a = nat.LayerArgs()
-    a.ep_size, a.num_local_tokens, a.topk, a.num_local_experts = ep, T, K, E
+    a.ep_size, a.num_local_tokens, a.topk, a.num_local_experts, a.hidden, a.intermediate = ep, T, K, E, H, I
     return nat, a
 
 
@@ -21,19 +21,26 @@ def test_scratch_of_the_mxfp8_calls(monkeypatch, ep, env, act, grad):
     assert nat.lib().mok_layer_scratch(nat.ctypes.byref(a), 1) == want
 
 
-@pytest.mark.parametrize("T,K,E,partials", [(512, 8, 32, True), (512, 8, 31, False)])
-def test_row_partials_of_the_bf16_backward(monkeypatch, T, K, E, partials):
-    nat, a = _args(T, K, E)
+@pytest.mark.parametrize("T,K,E,H,I,partials", [(512, 8, 64, 2048, 2048, True),      # 64 rows per expert, 512 MB of weights
+                                                (768, 8, 95, 2048, 2048, False),     # a little more than 64
+                                                (512, 8, 128, 2048, 512, True),      # 256 MB, twice the L2
+                                                (512, 8, 127, 2048, 512, False), (512, 1, 1024, 7168, 2048, True)])
+def test_padding_left_out_and_row_partials_of_the_bf16_calls(monkeypatch, T, K, E, H, I, partials):
+    nat, a = _args(T, K, E, H=H, I=I)
     always = nat.SCRATCH_DISPATCHED | nat.SCRATCH_ACTIVATIONS | nat.SCRATCH_GRADIENTS
-    assert nat.lib().mok_layer_scratch(nat.ctypes.byref(a), 0) == always | (nat.SCRATCH_ROW_PARTIALS if partials else 0)
+    used = lambda: nat.lib().mok_layer_scratch(nat.ctypes.byref(a), 0)  # noqa: E731
+    assert used() == always | (nat.SCRATCH_ROW_PARTIALS if partials else 0)
     monkeypatch.setenv("MOK_NO_ROW_TRIM", "1")
-    assert nat.lib().mok_layer_scratch(nat.ctypes.byref(a), 0) == always
+    assert used() == always
+    monkeypatch.setenv("MOK_NO_ROW_TRIM", "0")
+    assert used() == always | nat.SCRATCH_ROW_PARTIALS
 
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("E,partials", [(4, False), (16, True)])
-def test_memory_beyond_the_outputs(E, partials):
+def test_memory_beyond_the_outputs(monkeypatch, E, partials):
     import mok
+    monkeypatch.setenv("MOK_NO_ROW_TRIM", "0" if partials else "1")
     ops, dev = mok.ops, torch.device("cuda", 0)
     T, H, I, K, MB = 512, 1024, 1024, 2, 16384
     g = torch.Generator(device=dev).manual_seed(8)

@@ -63,8 +63,9 @@ def _fixed_capacity(sched, rows_per_expert, length):
 @pytest.mark.gpu
 @pytest.mark.parametrize("mxfp8", [False, True])
 @pytest.mark.parametrize("skip", [False, True])                      # rows kept, or stored into the slots by the epilogue
-@pytest.mark.parametrize("T,K,E,pad,MB", [(1536, 2, 5, 0, 8192), (1536, 2, 5, 0, 2560), (768, 2, 21, 0, 8192), (768, 2, 13, 512, 8192)])
-def test_layer_is_the_same_for_every_group_width(monkeypatch, mxfp8, skip, T, K, E, pad, MB):
+@pytest.mark.parametrize("T,K,E,pad,MB,no_trim", [(1536, 2, 5, 0, 8192, "1"), (1536, 2, 5, 0, 2560, "1"), (768, 2, 21, 0, 8192, "0"),
+                                                  (768, 2, 13, 512, 8192, "0")])
+def test_layer_is_the_same_for_every_group_width(monkeypatch, mxfp8, skip, T, K, E, pad, MB, no_trim):
     """Fused, dual, scattered, routed and MXFP8 rows forms: bitwise what m tile major order gives, with ragged experts, several
     windows, a last group that is narrower than the others and tiles that hold padding only."""
     import mok
@@ -106,6 +107,7 @@ def test_layer_is_the_same_for_every_group_width(monkeypatch, mxfp8, skip, T, K,
         ops.check_status(dev)
         return [slots, d_slots, d_rw, *grads]
 
+    monkeypatch.setenv("MOK_NO_ROW_TRIM", no_trim)
     monkeypatch.setenv("MOK_ROWS_GROUP", "1")
     want = run()
     for width in ("4", "8"):
