@@ -39,7 +39,7 @@ struct KernelParams {
     bf16* D0;
     bf16* D1;
     bf16* D2;                 // bf16 kernel, fused gate / up form: hidden = silu(gate) * up (D0 = gate, D1 = up)
-    const bf16* gate;         // routed bf16 kernel, SwiGLU backward: saved gate / up (D0 = d_hidden or nullptr, D1 = d_gate, D2 = d_up)
+    const bf16* gate;         // routed bf16 kernel, SwiGLU backward: saved gate / up (D0 = d_hidden, D1 = d_gate, D2 = d_up)
     const bf16* up;
     float* row_partial;       // and per row and 128 columns the sum of d_hidden * hidden, [rows, N / 128], or nullptr
     int clamp;                // fused SwiGLU forms: clamp on
@@ -252,6 +252,14 @@ inline int encode_map(CUtensorMap* map, CUtensorMapDataType type, const void* ba
         return MOK_ERR_CUDA;
     }
     return MOK_OK;
+}
+
+// Rank-4 bf16 map over a row-major [d2][d1][d0] array (d0 contiguous); box = {b0, b1, 1, 1}.
+inline int make_map(CUtensorMap* map, const void* base, uint64_t d0, uint64_t d1, uint64_t d2, uint32_t b0, uint32_t b1) {
+    const cuuint64_t dims[4] = {d0, d1, d2, 1};
+    const cuuint64_t strides[3] = {d0 * 2, d0 * d1 * 2, d0 * d1 * d2 * 2};
+    const cuuint32_t box[4] = {b0, b1, 1, 1};
+    return encode_map(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, base, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B);
 }
 
 inline int check_problem(const GemmProblem& pb) {

@@ -23,6 +23,7 @@
 // to bf16, stores them (backward needs them) and forms hidden = silu(gate) * up from the rounded values, which is
 // exactly what a separate SwiGLU pass over the stored gate / up would compute, without reading them back.
 #include "gemm_tiles.cuh"
+#include "routed_gemm.cuh"
 #include "swiglu_math.cuh"
 
 namespace mok {
@@ -323,14 +324,6 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_const
 // Host side
 // ---------------------------------------------------------------------------------------------------------
 
-// Rank-4 bf16 map over a row-major [d2][d1][d0] array (d0 contiguous); box = {b0, b1, 1, 1}.
-int make_map(CUtensorMap* map, const void* base, uint64_t d0, uint64_t d1, uint64_t d2, uint32_t b0, uint32_t b1) {
-    const cuuint64_t dims[4] = {d0, d1, d2, 1};
-    const cuuint64_t strides[3] = {d0 * 2, d0 * d1 * 2, d0 * d1 * d2 * 2};
-    const cuuint32_t box[4] = {b0, b1, 1, 1};
-    return encode_map(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, base, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B);
-}
-
 size_t smem_bytes(int num_experts) {
     return 1024 + SharedLayout::kCum + 4 * (static_cast<size_t>(num_experts) + 2);
 }
@@ -345,14 +338,6 @@ int launch(const CUtensorMap& a0, const CUtensorMap& b0, const CUtensorMap& a1, 
 
 
 }  // namespace
-
-// routed_gemm.cu: the rows forms for problems that know their occupied rows (arguments already checked)
-int launch_routed_gemm(const GemmProblem& pb, const void* A0, const void* A1, int K, const void* B0, const void* B1, void* D, int N,
-                       bool b_is_kn, cudaStream_t stream, const RowScatter* scatter);
-int launch_routed_gate_up(const GemmProblem& pb, const void* A, int K, const void* Wg, const void* Wu, void* gate, void* up, void* hidden,
-                          int N, bool has_limit, float limit, cudaStream_t stream);
-int launch_routed_down_dgrad(const GemmProblem& pb, const void* A, int K, const void* B, const void* gate, const void* up, void* d_hidden,
-                             void* d_gate, void* d_up, float* row_partial, int N, bool has_limit, float limit, cudaStream_t stream);
 
 int launch_rows_gemm(const GemmProblem& pb, const void* A, int K, const void* B0, const void* B1, void* D0, void* D1,
                      int N, bool b_is_kn, cudaStream_t stream, const RowScatter* scatter) {
@@ -412,7 +397,8 @@ int launch_gate_up_fused(const GemmProblem& pb, const void* A, int K, const void
 int launch_down_dgrad_fused(const GemmProblem& pb, const void* A, int K, const void* B, const void* gate, const void* up, void* d_hidden,
                             void* d_gate, void* d_up, float* row_partial, int N, bool has_limit, float limit, cudaStream_t stream) {
     if (int rc = check_problem(pb)) return rc;
-    if (K <= 0 || N <= 0 || K % BK != 0 || N % BN != 0 || !gate || !up || !d_gate || !d_up || !pb.occupied_rows) return MOK_ERR_INVALID_ARGUMENT;
+    if (K <= 0 || N <= 0 || K % BK != 0 || N % BN != 0 || !gate || !up || !d_hidden || !d_gate || !d_up || !pb.occupied_rows)
+        return MOK_ERR_INVALID_ARGUMENT;
     return launch_routed_down_dgrad(pb, A, K, B, gate, up, d_hidden, d_gate, d_up, row_partial, N, has_limit, limit, stream);
 }
 

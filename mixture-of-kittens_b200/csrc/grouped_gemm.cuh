@@ -37,7 +37,8 @@ struct RowScatter {
 };
 
 // D_s[row, :] = A[row, :K] * B_s[e]^T for s < n_sets (two sets share A: gate and up projections).
-// With `scatter` (one set only) D0 is nullptr and the rows go to their slots.  b_is_kn = false: B_s is [E, N, K];  true: B_s is [E, K, N].
+// With `scatter` (one set only) D0 is nullptr and the rows go to their slots.
+// b_is_kn = false: B_s is [E, N, K];  true: B_s is [E, K, N].
 int launch_rows_gemm(const GemmProblem& pb, const void* A, int K, const void* B0, const void* B1, void* D0, void* D1,
                      int N, bool b_is_kn, cudaStream_t stream, const RowScatter* scatter = nullptr);
 
@@ -47,7 +48,7 @@ int launch_gate_up_fused(const GemmProblem& pb, const void* A, int K, const void
                          void* hidden, int N, bool has_limit, float limit, cudaStream_t stream);
 
 // Input gradient of the down projection with the SwiGLU backward in the epilogue: d_hidden = A * B[e] (B stored [E, K, N])
-// rounded to bf16 and stored (unless nullptr), d_gate / d_up from it and the saved gate / up [rows, N].
+// rounded to bf16 and stored, d_gate / d_up from it and the saved gate / up [rows, N].
 // row_partial (or nullptr): [rows, N / 128] sums of d_hidden * hidden for the router-weight gradient (launch_router_grad).
 // Needs pb.occupied_rows.
 int launch_down_dgrad_fused(const GemmProblem& pb, const void* A, int K, const void* B, const void* gate, const void* up, void* d_hidden,

@@ -135,7 +135,10 @@ bool gathers_in_quantizer(const mok_layer_args* a);
 
 // see mok_layer_scratch
 unsigned scratch_used(const mok_layer_args* a, bool fp8) {
-    if (!fp8) return MOK_SCRATCH_DISPATCHED | MOK_SCRATCH_ACTIVATIONS | MOK_SCRATCH_GRADIENTS | (row_trim_enabled(a) ? MOK_SCRATCH_ROW_PARTIALS : 0u);
+    if (!fp8) {
+        const unsigned outputs = MOK_SCRATCH_DISPATCHED | MOK_SCRATCH_ACTIVATIONS | MOK_SCRATCH_GRADIENTS;
+        return outputs | (row_trim_enabled(a) ? MOK_SCRATCH_ROW_PARTIALS : 0u);
+    }
     unsigned used = 0;
     if (!gathers_in_quantizer(a)) used |= MOK_SCRATCH_DISPATCHED;
     if (!fused_activations_enabled() || !fused_epilogue_enabled()) used |= MOK_SCRATCH_ACTIVATIONS;
@@ -851,8 +854,7 @@ extern "C" int mok_moe_backward_mxfp8(const mok_layer_args* a, mok_stream_t stre
     float* row_grad = a->row_scratch + a->macrobatch_size;
     const long long sc_I = scale_tile_row_bytes(I);
     int32_t* occupied = occupied_rows_of(a);
-    MOK_TRY(launch_occupied_rows(a->peer_rank, a->tokens_per_expert, a->num_tokens, a->schedule_capacity, a->num_local_experts,
-                                 occupied, s));
+    MOK_TRY(find_occupied_rows(a, occupied, s));
     for (int wi = 0; wi < num_windows(a); ++wi) {
         const Span win = window_span(a, wi);
         if (wi > 0) {

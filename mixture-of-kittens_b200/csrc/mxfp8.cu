@@ -117,8 +117,9 @@ __device__ __forceinline__ void copy_async_wait() { asm volatile("cp.async.wait_
 // Bound by HBM.  A block walks `tiles_per_block` column tiles of one row tile; the next tile is on its way into the second
 // buffer while one is being quantized.  One tile per block and plain loads left the block waiting for its own loads two
 // thirds of the time, whatever the order of the tiles: 37k gathered rows of 7168 359 us (242 us with the leaner arithmetic
-// and 6 instead of 4 resident blocks), now 197 us (5.5 TB/s); weights 32 x 2048 x 7168 441 -> 419 us.  16 lanes per row and eight consecutive columns per lane, eight rows per thread: a block of 32 along the row is four adjacent lanes,
-// so the normal layout is quantized from registers (mxfp8_quantize_quarter) and stored as full 128-byte lines.
+// and 6 instead of 4 resident blocks), now 197 us (5.5 TB/s); weights 32 x 2048 x 7168 441 -> 419 us.  16 lanes per row and
+// eight consecutive columns per lane, eight rows per thread: a block of 32 along the row is four adjacent lanes, so the normal
+// layout is quantized from registers (mxfp8_quantize_quarter) and stored as full 128-byte lines.
 // GATHER: the tile's rows are schedule rows whose tokens are read where they lie (`x` = all tokens of this rank), and
 // with weights scaled on the way, instead of from a buffer that a dispatch pass has filled.
 constexpr int kQuantThreads = 256;
@@ -206,9 +207,9 @@ __global__ void __launch_bounds__(kQuantThreads, kQuantBlocksPerSm) quantize_ker
 
 // ---- fused activation steps ---------------------------------------------------------------------------------------
 // Both kernels walk a 128 x 128 tile with 16 lanes per row and eight consecutive columns per lane, sixteen rows per
-// thread: a block of 32 along the row is four adjacent lanes, so the normal layout is quantized straight from
-// registers (mxfp8_quantize_quarter) and stored as full 128-byte lines; the values that also need the transposed
-// layout go through the shared-memory tile.
+// thread in the forward (128 threads) and eight in the backward (256): a block of 32 along the row is four adjacent lanes, so
+// the normal layout is quantized straight from registers (mxfp8_quantize_quarter) and stored as full 128-byte lines; the values
+// that also need the transposed layout go through a shared-memory tile.
 struct FusedFwdArgs {
     const bf16 *gate, *up;
     uint8_t *gate_q, *gate_sc, *up_q, *up_sc, *hidden_q, *hidden_sc, *hidden_qt, *hidden_sct;

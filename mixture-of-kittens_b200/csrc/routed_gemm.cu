@@ -14,6 +14,7 @@
 // epilogue costs a little more than it saves; row_trim_enabled() in layer.cu says where the line lies.
 // Needs GemmProblem::occupied_rows; dense problems and callers without it use grouped_gemm.cu.
 #include "gemm_tiles.cuh"
+#include "routed_gemm.cuh"
 #include "swiglu_math.cuh"
 
 namespace mok {
@@ -98,7 +99,8 @@ struct RoutedMaps {
 template <bool W_MN, int EPI>
 __global__ void __launch_bounds__(kThreads, 1)
 routed_gemm_kernel(const __grid_constant__ RoutedMaps m0, const __grid_constant__ RoutedMaps m1, const KernelParams p) {
-    static_assert(EPI == EPI_STORE || W_MN == (EPI == EPI_SWIGLU_BWD), "gate / up is a forward form, the SwiGLU backward an input gradient");
+    static_assert(EPI == EPI_STORE || W_MN == (EPI == EPI_SWIGLU_BWD),
+                  "gate / up is a forward form, the SwiGLU backward an input gradient");
     extern __shared__ uint8_t smem_raw[];
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t* smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
@@ -320,7 +322,7 @@ routed_gemm_kernel(const __grid_constant__ RoutedMaps m0, const __grid_constant_
                             }
                             uint4 dg, du;
                             float sum = p.clamp ? swiglu_bwd_vec<true>(g, u, w, p.limit, dg, du) : swiglu_bwd_vec<false>(g, u, w, 0.f, dg, du);
-                            if (p.D0 != nullptr) *reinterpret_cast<uint4*>(p.D0 + off) = w;
+                            *reinterpret_cast<uint4*>(p.D0 + off) = w;
                             *reinterpret_cast<uint4*>(p.D1 + off) = dg;
                             *reinterpret_cast<uint4*>(p.D2 + off) = du;
 #pragma unroll
@@ -343,7 +345,7 @@ routed_gemm_kernel(const __grid_constant__ RoutedMaps m0, const __grid_constant_
                 const uint4 zero = make_uint4(0, 0, 0, 0);
                 for (int r = n + group * 4 * kRowsPerWarp + sub; r < BN; r += 8 * kRowsPerWarp) {
                     const long long off = first + static_cast<long long>(r) * p.ldd;
-                    if (p.D0 != nullptr) *reinterpret_cast<uint4*>(p.D0 + off) = zero;
+                    *reinterpret_cast<uint4*>(p.D0 + off) = zero;
                     if (EPI != EPI_STORE) {
                         *reinterpret_cast<uint4*>(p.D1 + off) = zero;
                         *reinterpret_cast<uint4*>(p.D2 + off) = zero;
@@ -366,14 +368,6 @@ routed_gemm_kernel(const __grid_constant__ RoutedMaps m0, const __grid_constant_
         tc_fence_after_sync();
         tmem_dealloc_pair(tmem_base, TMEM_COLS);
     }
-}
-
-// Rank-4 bf16 map over a row-major [d2][d1][d0] array (d0 contiguous); box = {b0, b1, 1, 1}.
-int make_map(CUtensorMap* map, const void* base, uint64_t d0, uint64_t d1, uint64_t d2, uint32_t b0, uint32_t b1) {
-    const cuuint64_t dims[4] = {d0, d1, d2, 1};
-    const cuuint64_t strides[3] = {d0 * 2, d0 * d1 * 2, d0 * d1 * d2 * 2};
-    const cuuint32_t box[4] = {b0, b1, 1, 1};
-    return encode_map(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, base, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B);
 }
 
 template <bool W_MN, int EPI>
@@ -403,7 +397,6 @@ int tiles_of(const GemmProblem& pb, const KernelParams& kp) { return ((pb.row_en
 
 }  // namespace
 
-// The callers (grouped_gemm.cu) have checked the problem and the sizes.
 int launch_routed_gemm(const GemmProblem& pb, const void* A0, const void* A1, int K, const void* B0, const void* B1, void* D, int N,
                        bool b_is_kn, cudaStream_t stream, const RowScatter* scatter) {
     RoutedMaps m0, m1;

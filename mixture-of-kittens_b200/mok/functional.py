@@ -283,7 +283,8 @@ def _scatter_from_gemm(workspace: MoKWorkspace) -> bool:
     """Whether the down projection and the input-gradient GEMM store their rows into the combine slots themselves instead
     of leaving them to a combine pass (the results are the same).  On for one rank, where it saves a read and a write of
     every row (DeepSeek-V3-shaped layer, 32 experts: training step of 32768 tokens in bf16 79.6 -> 77.0 ms, of 16384 tokens
-    in MXFP8 30.9 -> 29.4 ms; Qwen3-MoE-shaped forward of 512 tokens 420 -> 378 us).  With several ranks the combine pass overlaps the NVLink stores with the GEMMs of the next chunk; that order is the measured one."""
+    in MXFP8 30.9 -> 29.4 ms; Qwen3-MoE-shaped forward of 512 tokens 425 -> 378 us).  With several ranks the combine pass
+    overlaps the NVLink stores with the GEMMs of the next chunk; that order is the measured one."""
     return workspace.ep_size == 1
 
 
