@@ -245,18 +245,22 @@ bool fused_swiglu_enabled() {
 // (routed_gemm.cu), with the SwiGLU backward in the epilogue of the input gradient.  An expert is padded to 256 rows, so with
 // few rows each most rows are padding.  The gain is there while the GEMMs wait for weights from HBM; the price is a launch more
 // in the forward and an epilogue that transposes, 2 to 10 us a call and more for full tiles, which skewed loads have too.  Time
-// with the padding / without (forward, forward + backward; balanced and Zipf(1.2) loads; L2 flushed), by average rows per expert
-// and by the bytes of one projection's weights in all experts:
-//   hidden x intermediate x experts        32 balanced   32 Zipf       64 balanced   64 Zipf       128 balanced  128 Zipf
-//   2048 x  768 x 128  (402 MB)            1.050 1.051   1.012 1.009   1.036 1.036   0.987 1.027   0.990 0.998   1.005 1.020
-//   4096 x 1024 x 128 (1074 MB)            1.074 1.059   1.035 1.026   1.061 1.046   1.040 1.037
-//   4096 x 1536 x  64  (805 MB)            1.050 1.041   1.035 1.019   1.032 1.021   1.019 1.027
-//   7168 x 2048 x 128 (3758 MB)            1.013 1.042   1.016 1.029   0.984 1.008   1.000 1.011   0.879 0.939   0.960 1.003
-//   7168 x 2048 x  16  (470 MB)            1.017 1.014   1.020 1.010   0.995 0.999   1.020 1.016
-//   2048 x  768 x  64  (201 MB)            1.034 1.043   0.990 0.986   1.008 1.019   1.000 0.990
+// with the padding / without (forward, forward + backward; balanced and Zipf(1.2) loads; L2 flushed; runs differ by 0.01 to
+// 0.04), by average rows per expert and by the bytes of one projection's weights in all experts:
+//   hidden x intermediate x experts        32 balanced   32 Zipf       64 balanced   64 Zipf       96 balanced   128 balanced
+//   2048 x  768 x 128  (402 MB)            1.050 1.051   1.012 1.009   1.036 1.036   0.987 1.027   1.011 1.021   0.990 0.998
+//   4096 x 1024 x 128 (1074 MB)            1.074 1.059   1.035 1.026   1.061 1.046   1.040 1.037   1.040 1.016   0.945 0.986
+//   4096 x 1536 x  64  (805 MB)            1.050 1.041   1.035 1.019   1.032 1.021   1.019 1.027   1.026 1.018   0.989 0.979
+//   4096 x 2048 x  32  (537 MB)            1.037 1.036   0.996 1.007   1.021 1.027   1.020 1.022   1.014 1.017   0.989 0.990
+//   7168 x 2048 x 128 (3758 MB)            1.013 1.042   1.016 1.029   1.008 1.011   0.991 1.034   0.947 0.968   0.879 0.939
+//   7168 x 2048 x  16  (470 MB)            1.017 1.014   1.020 1.010   0.995 0.999   1.020 1.016   0.992 0.999
+//   1024 x  768 x 128  (201 MB)            1.053 1.039   0.966 0.991   1.053 1.032   0.966 0.978
+//   2048 x  768 x  64  (201 MB)            1.019 1.017   0.989 0.994   0.997 1.008   0.990 1.007   0.983 1.009
 //   1024 x  512 x 128  (134 MB)            1.068 1.015   0.960 0.970   1.022 1.013   0.938 0.979
-//   1024 x  512 x  64   (67 MB)            1.014 0.994   0.944 0.961   1.014 0.999   0.943 0.969   0.937 0.976   0.948 0.957
-// So: at most 64 rows on average, and weights that outgrow the 126 MB L2 twice.
+//   1024 x  512 x  64   (67 MB)            1.014 0.994   0.944 0.961   1.014 0.999   0.943 0.969                 0.937 0.976
+//   2048 x 1024 x  16   (67 MB)            0.985 1.007   0.984 0.985   0.972 0.979   0.988 0.974
+// So: at most 96 rows on average, 64 above hidden 4096, and weights that do not fit the 126 MB L2.  Between there and 256 MB a
+// Zipf load costs 2 to 10 us that ordinary loads gain; the loads are not known on the host.
 // MOK_NO_ROW_TRIM=1 computes the padding rows always, =0 never; the results are the same but for the order in which the
 // router-weight gradient is summed.
 bool row_trim_enabled(const mok_layer_args* a) {
@@ -264,8 +268,9 @@ bool row_trim_enabled(const mok_layer_args* a) {
         if (v[0] == '1') return false;
         if (v[0] == '0') return true;
     }
-    return static_cast<long long>(a->num_local_tokens) * a->topk <= 64LL * a->num_local_experts &&
-           2LL * a->num_local_experts * a->hidden * a->intermediate >= (256LL << 20);
+    const long long rows = a->hidden <= 4096 ? 96 : 64;
+    return static_cast<long long>(a->num_local_tokens) * a->topk <= rows * a->num_local_experts &&
+           2LL * a->num_local_experts * a->hidden * a->intermediate >= (126LL << 20);
 }
 
 // MOK_NO_WGRAD_TRIM=1 lets the weight-gradient GEMMs run over the padding rows too (for measurements; same results)

@@ -21,10 +21,12 @@ def test_scratch_of_the_mxfp8_calls(monkeypatch, ep, env, act, grad):
     assert nat.lib().mok_layer_scratch(nat.ctypes.byref(a), 1) == want
 
 
-@pytest.mark.parametrize("T,K,E,H,I,partials", [(512, 8, 64, 2048, 2048, True),      # 64 rows per expert, 512 MB of weights
-                                                (768, 8, 95, 2048, 2048, False),     # a little more than 64
-                                                (512, 8, 128, 2048, 512, True),      # 256 MB, twice the L2
-                                                (512, 8, 127, 2048, 512, False), (512, 1, 1024, 7168, 2048, True)])
+@pytest.mark.parametrize("T,K,E,H,I,partials", [(768, 8, 64, 4096, 1024, True),      # 96 rows per expert
+                                                (768, 8, 63, 4096, 1024, False),     # a little more
+                                                (512, 8, 64, 4352, 1024, True),      # 64 rows per expert above hidden 4096
+                                                (512, 8, 63, 4352, 1024, False),
+                                                (512, 8, 126, 1024, 512, True),      # 126 MB of weights, what the L2 holds
+                                                (512, 8, 125, 1024, 512, False), (512, 1, 1024, 7168, 2048, True)])
 def test_padding_left_out_and_row_partials_of_the_bf16_calls(monkeypatch, T, K, E, H, I, partials):
     nat, a = _args(T, K, E, H=H, I=I)
     always = nat.SCRATCH_DISPATCHED | nat.SCRATCH_ACTIVATIONS | nat.SCRATCH_GRADIENTS
