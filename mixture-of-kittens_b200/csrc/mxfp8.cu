@@ -1,5 +1,5 @@
 // MXFP8 quantizer: bf16 -> e4m3 elements with one e8m0 scale per 32 elements along the row, for a matrix and /
-// or its transpose.  HBM-bound: one 128 x 128 tile per CTA is staged in shared memory once and both layouts are
+// or its transpose.  HBM-bound: every 128 x 128 tile is staged in shared memory once and both layouts are
 // produced from it (2 B read, up to 2 x 1.03 B written per element).
 //
 // Arithmetic (bit-exact with the reference device code, csrc/mxfp8.cuh:45-72): scale = max(amax * fp32(1/448),
@@ -117,9 +117,9 @@ __device__ __forceinline__ void copy_async_wait() { asm volatile("cp.async.wait_
 // Bound by HBM.  A block walks `tiles_per_block` column tiles of one row tile; the next tile is on its way into the second
 // buffer while one is being quantized.  One tile per block and plain loads left the block waiting for its own loads two
 // thirds of the time, whatever the order of the tiles: 37k gathered rows of 7168 359 us (242 us with the leaner arithmetic
-// and 6 instead of 4 resident blocks), now 197 us (5.5 TB/s); weights 32 x 2048 x 7168 441 -> 419 us.  16 lanes per row and
-// eight consecutive columns per lane, eight rows per thread: a block of 32 along the row is four adjacent lanes, so the normal
-// layout is quantized from registers (mxfp8_quantize_quarter) and stored as full 128-byte lines.
+// and 6 instead of 4 resident blocks), now 197 us (5.5 TB/s); weights 32 x 2048 x 7168 in both layouts 395 -> 340 us.
+// 16 lanes per row and eight consecutive columns per lane, eight rows per thread: a block of 32 along the row is four adjacent
+// lanes, so the normal layout is quantized from registers (mxfp8_quantize_quarter) and stored as full 128-byte lines.
 // GATHER: the tile's rows are schedule rows whose tokens are read where they lie (`x` = all tokens of this rank), and
 // with weights scaled on the way, instead of from a buffer that a dispatch pass has filled.
 constexpr int kQuantThreads = 256;
