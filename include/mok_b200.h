@@ -42,7 +42,10 @@ enum {
 #define MOK_MAX_EP 8
 #define MOK_MAX_LOCAL_EXPERTS 1024
 
-/* Library/ABI version (major*100+minor); also proves the library loaded. */
+/* Library/ABI version (major*100+minor); also proves the library loaded.  It changes whenever mok_layer_args does: a program that
+ * was compiled against another version's header must not pass its struct, whose end the library would read past.
+ * 101: schedule_rows (was reserved1), occupied_rows, row_partials; NULL y_routed / d_x_routed; mok_layer_scratch. */
+#define MOK_VERSION 101
 int mok_version(void);
 
 /* Last CUDA error string seen by this library on the calling thread ("" if none). */

@@ -35,7 +35,7 @@ int sm_count() {
 
 }  // namespace mok
 
-extern "C" int mok_version(void) { return 100; }
+extern "C" int mok_version(void) { return MOK_VERSION; }
 
 extern "C" const char* mok_last_error(void) { return mok::g_last_error; }
 

@@ -23,6 +23,7 @@ STATUS_BITS = {
     8: "a schedule row named a peer or token outside the buffers, or the schedule claims more rows than were promised",
 }
 MAX_EP = 8
+VERSION = 101   # MOK_VERSION of the header that LayerArgs mirrors
 # MOK_SCRATCH_* bits of mok_layer_scratch
 SCRATCH_DISPATCHED, SCRATCH_ACTIVATIONS, SCRATCH_GRADIENTS, SCRATCH_ROW_PARTIALS = 1, 2, 4, 8
 
@@ -61,6 +62,9 @@ def lib() -> ctypes.CDLL:
                               "there is no fallback implementation")
         L = ctypes.CDLL(_LIB_PATH)
         L.mok_version.restype = c_int
+        if L.mok_version() != VERSION:
+            raise ImportError(f"{_LIB_PATH} has ABI version {L.mok_version()}, this package expects {VERSION}: build it again with "
+                              "`python mixture-of-kittens_b200/build.py`")
         L.mok_last_error.restype = c_char_p
         L.mok_launch_count.restype = ctypes.c_longlong
         L.mok_schedule_scratch_bytes.restype = c_int64

@@ -60,6 +60,19 @@ def test_layer_args_struct_matches_header_field_order():
     assert names == [f[0] for f in nat.LayerArgs._fields_]
 
 
+def test_version_of_header_library_and_package_agree(monkeypatch):
+    from mok import _native as nat
+    header = open(os.path.join(ROOT, "include", "mok_b200.h")).read()
+    version = int(re.search(r"#define MOK_VERSION (\d+)", header).group(1))
+    assert nat.lib().mok_version() == version == nat.VERSION
+    # the struct is what the version stands for: both change together
+    assert (version, nat.ctypes.sizeof(nat.LayerArgs)) == (101, 768)
+    monkeypatch.setattr(nat, "_lib", None)
+    monkeypatch.setattr(nat, "VERSION", version + 1)
+    with pytest.raises(ImportError, match="ABI version"):
+        nat.lib()
+
+
 def test_python_surface_mirrors_the_reference_interface():
     import mok
     F = mok.functional
